@@ -2,7 +2,9 @@
 // (src/filters/gaussian.rs:74-88) that runs one convolve_axis
 // (src/filters/conv.rs:11-41) per axis through an f32 scratch buffer.  It
 // covers every dimension, dtype, component count and radius up to 384, and is
-// the fallback when no fused kernel fits.
+// the fallback when no fused kernel fits.  From radius 8 on the passes of
+// conv_lines.cu take over (except along x into another type, which only 1-D
+// images need); what stays here are the shorter kernels and small images.
 //
 // One thread computes one output component; threads run along axis 0 so loads
 // and stores coalesce for every pass (for axes 1 and 2 each tap is a row-wide
@@ -134,7 +136,7 @@ __global__ void __launch_bounds__(kThreads)
 // zero, clamp to [lo, hi] on `axis`.
 template <int R>
 constexpr int run_of() { return R <= 2 ? 8 : 4; }
-constexpr int kMaxSmallR = 12;
+constexpr int kMaxSmallR = kMaxSmallRadius;
 
 template <int R, bool REF>
 __global__ void __launch_bounds__(kThreads, R <= 4 ? 4 : 2)
@@ -285,6 +287,8 @@ itkg_status launch_conv_axis_f32(const AxisArgs& a, const float* w, int in_dtype
     return set_error(ITKG_ERROR_UNSUPPORTED, "radius %d exceeds the per-axis limit %d", a.radius,
                      (kMaxParamTaps - 1) / 2);
   if (a.out_size[0] * a.out_size[1] * a.out_size[2] == 0) return ITKG_SUCCESS;
+  const itkg_status st = launch_conv_lines(a, w, in_dtype, out_dtype, rounding, stream);
+  if (st != ITKG_ERROR_UNSUPPORTED) return st;
   AxisWeightsF32 W;
   for (int k = 0; k < K; ++k) W.w[k] = w[k];
   for (int k = K; k < kMaxParamTaps; ++k) W.w[k] = 0.0f;

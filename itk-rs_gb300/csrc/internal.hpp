@@ -70,6 +70,14 @@ struct AxisWeightsF64 {  // u8 pixel path: exact f64 weights
 // conv_axis.cu
 itkg_status launch_conv_axis_f32(const AxisArgs& a, const float* w, int in_dtype,
                                  int out_dtype, int rounding, void* stream);
+// Largest radius of conv_axis.cu's unrolled f32 -> f32 pass.
+constexpr int kMaxSmallRadius = 12;
+// conv_lines.cu: the same pass for runs of 16 outputs per thread; needs
+// 2 radius >= 15 (and, up to kMaxSmallRadius between f32 images, a grid that
+// occupies the chip) and an f32 output along x, an f32 input along y and z.
+// ITKG_ERROR_UNSUPPORTED (no error set) when it does not apply.
+itkg_status launch_conv_lines(const AxisArgs& a, const float* w, int in_dtype, int out_dtype, int rounding,
+                              void* stream);
 // lut_buf: 256-byte aligned device buffer of at least (2 radius + 1) * 256
 // bytes for the per-tap table, or NULL to take it from scratch_alloc.  The
 // table kernel and the filter kernel run in order on `stream`, so one buffer
