@@ -31,17 +31,23 @@ struct RecGeom {
   int64_t lo[3];       // largest region index
 };
 
-template <typename Tin, typename T>
-__global__ void __launch_bounds__(kT) k_rec_load(const char* src, int64_t so0, int64_t so1, int64_t so2,
-                                                  int64_t sp0, int64_t sp1, int64_t sp2, RecGeom g, T* d) {
-  const int64_t x = (int64_t)blockIdx.x * kT + threadIdx.x;
-  if (x >= g.n[0]) return;
-  for (int64_t z = blockIdx.z; z < g.n[2]; z += gridDim.z)
-    for (int64_t y = blockIdx.y; y < g.n[1]; y += gridDim.y) {
-      const char* p = src + (g.lo[0] + x - so0) * sp0 + (g.lo[1] + y - so1) * sp1 + (g.lo[2] + z - so2) * sp2;
-      const float v = to_f32(*reinterpret_cast<const Tin*>(p));  // exact for every input type
-      d[(z * g.n[1] + y) * g.n[0] + x] = (T)v;
-    }
+// An input or output image seen from the largest region: byte strides per axis,
+// the address of the largest region's first voxel.
+struct RecImage {
+  char* at;
+  int64_t p[3];
+  int32_t dtype;
+  int32_t pad_;
+};
+
+__device__ __forceinline__ double rec_read(const char* p, int dtype) {  // exact for every input type
+  switch (dtype) {
+    case ITKG_F32: return (double)*reinterpret_cast<const float*>(p);
+    case ITKG_I16: return (double)to_f32(*reinterpret_cast<const int16_t*>(p));
+    case ITKG_U8: return (double)to_f32(*reinterpret_cast<const uint8_t*>(p));
+    case ITKG_BF16: return (double)to_f32(*reinterpret_cast<const __nv_bfloat16*>(p));
+    default: return (double)to_f32(*reinterpret_cast<const __half*>(p));
+  }
 }
 
 // v = B x + a1 y[-1] + a2 y[-2] + a3 y[-3]
@@ -58,51 +64,6 @@ __device__ __forceinline__ double rec_step(double x, double y1, double y2, doubl
   }
 }
 
-// One line per thread.  axis 0: lines are rows (stride 1); axis 1: stride n0;
-// axis 2: stride n0 n1.
-template <typename T, bool REF>
-__global__ void __launch_bounds__(kT) k_rec_lines(T* d, RecGeom g, int axis, T B, T a1, T a2, T a3) {
-  const int64_t L = (int64_t)blockIdx.x * kT + threadIdx.x;
-  const int64_t n0 = g.n[0], n1 = g.n[1], n2 = g.n[2];
-  int64_t nlines, base, s, n;
-  if (axis == 0) {
-    nlines = n1 * n2;
-    base = L * n0;
-    s = 1;
-    n = n0;
-  } else if (axis == 1) {
-    nlines = n0 * n2;
-    base = (L / n0) * n0 * n1 + L % n0;
-    s = n0;
-    n = n1;
-  } else {
-    nlines = n0 * n1;
-    base = L;
-    s = n0 * n1;
-    n = n2;
-  }
-  if (L >= nlines) return;
-  T* const p = d + base;
-  T y1 = p[0], y2 = y1, y3 = y1;  // steady state of the first sample
-  for (int64_t i = 0; i < n; ++i) {
-    const T v = rec_step<REF>(p[i * s], y1, y2, y3, B, a1, a2, a3);
-    y3 = y2;
-    y2 = y1;
-    y1 = v;
-    p[i * s] = v;
-  }
-  y1 = p[(n - 1) * s];
-  y2 = y1;
-  y3 = y1;
-  for (int64_t i = n - 1; i >= 0; --i) {
-    const T v = rec_step<REF>(p[i * s], y1, y2, y3, B, a1, a2, a3);
-    y3 = y2;
-    y2 = y1;
-    y1 = v;
-    p[i * s] = v;
-  }
-}
-
 __device__ __forceinline__ float out_f32(double v) { return __double2float_rn(v); }
 __device__ __forceinline__ uint8_t out_u8_of(double v) {  // round half away from zero, clamp, NaN -> 0
   double r = round(v);
@@ -110,20 +71,147 @@ __device__ __forceinline__ uint8_t out_u8_of(double v) {  // round half away fro
   return (uint8_t)r;
 }
 
-template <typename T, int OUT>
-__global__ void __launch_bounds__(kT) k_rec_store(const T* d, RecGeom g, int64_t r0, int64_t r1, int64_t r2,
-                                                   int64_t m0, int64_t m1, int64_t m2, char* dst, int64_t do0,
-                                                   int64_t do1, int64_t do2, int64_t dp0, int64_t dp1, int64_t dp2) {
+__device__ __forceinline__ void rec_write(char* p, int dtype, double v) {
+  if (dtype == ITKG_U8) *reinterpret_cast<uint8_t*>(p) = out_u8_of(v);
+  else *reinterpret_cast<float*>(p) = out_f32(v);
+}
+
+struct RecLines {
+  RecGeom g;
+  double* d;            // scratch: sample (x, y, z) at (z n1 + y) pitch + x
+  int64_t pitch;        // doubles per row, a multiple of 4
+  int32_t axis;
+  int32_t pad_;
+  RecImage in, out;     // FIRST / LAST
+  int64_t in_step, out_step;  // their strides along the axis
+  int32_t w0, w1;       // LAST: the requested samples of a line
+  int64_t lo[3], hi[3]; // LAST: the requested region, from the largest one's first voxel
+  double B, a1, a2, a3;
+};
+
+// Four samples of a line, p[0], p[s], ...; CONTIG: s = 1 and p on a 16-byte
+// boundary.  n: how many exist (the rest repeat the last one that does).
+template <bool CONTIG>
+__device__ __forceinline__ void rec_load4(const double* p, int64_t s, int n, double (&v)[4]) {
+  if (CONTIG && n == 4) {
+    const double2 a = *reinterpret_cast<const double2*>(p), b = *reinterpret_cast<const double2*>(p + 2);
+    v[0] = a.x, v[1] = a.y, v[2] = b.x, v[3] = b.y;
+  } else {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[k] = p[min(k, n - 1) * s];
+  }
+}
+
+template <bool CONTIG>
+__device__ __forceinline__ void rec_store4(double* p, int64_t s, int n, const double (&v)[4]) {
+  if (CONTIG && n == 4) {
+    *reinterpret_cast<double2*>(p) = make_double2(v[0], v[1]);
+    *reinterpret_cast<double2*>(p + 2) = make_double2(v[2], v[3]);
+  } else {
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (k < n) p[k * s] = v[k];
+  }
+}
+
+// One line per thread.  axis 0: lines are rows (CONTIG); axis 1: stride pitch;
+// axis 2: stride n1 pitch.
+template <bool REF, bool FIRST, bool LAST, bool CONTIG>
+__global__ void __launch_bounds__(32) k_rec_lines(const __grid_constant__ RecLines a) {
+  const int64_t L = (int64_t)blockIdx.x * 32 + threadIdx.x;
+  const int64_t n0 = a.g.n[0], n1 = a.g.n[1], n2 = a.g.n[2];
+  int64_t c[3] = {0, 0, 0};  // the line's first voxel
+  if (CONTIG) {
+    c[1] = L % n1, c[2] = L / n1;
+  } else {
+    const int64_t q = L / n0;
+    c[0] = L - q * n0, c[1] = a.axis == 1 ? 0 : q, c[2] = a.axis == 1 ? q : 0;
+  }
+  if (CONTIG ? L >= n1 * n2 : L >= n0 * (a.axis == 1 ? n2 : n1)) return;
+  const int n = (int)(CONTIG ? n0 : a.axis == 1 ? n1 : n2);
+  const int64_t s = CONTIG ? 1 : a.axis == 1 ? a.pitch : a.pitch * n1;
+  double* const p = a.d + (c[2] * n1 + c[1]) * a.pitch + c[0];
+  const int64_t is = a.in_step, os = a.out_step;
+  const char* const ip = FIRST ? a.in.at + c[0] * a.in.p[0] + c[1] * a.in.p[1] + c[2] * a.in.p[2] : nullptr;
+  char* const op = LAST ? a.out.at + c[0] * a.out.p[0] + c[1] * a.out.p[1] + c[2] * a.out.p[2] : nullptr;
+  int w0 = 0, w1 = 0;  // samples to write
+  if (LAST) {
+    bool in = true;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) in = in && (d == a.axis || (c[d] >= a.lo[d] && c[d] < a.hi[d]));
+    if (in) w0 = a.w0, w1 = a.w1;
+  }
+  auto read = [&](int i, double (&v)[4]) {  // samples i .. i + 3 of the axis' input
+    const int m = min(4, n - i);
+    if constexpr (FIRST) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) v[k] = rec_read(ip + (int64_t)(i + min(k, m - 1)) * is, a.in.dtype);
+    } else {
+      rec_load4<CONTIG>(p + i * s, s, m, v);
+    }
+  };
+  double v[4], nx[4];
+  read(0, v);
+  double y1 = v[0], y2 = y1, y3 = y1;  // steady state of the first sample
+  for (int i = 0; i < n; i += 4) {
+    if (i + 4 < n) read(i + 4, nx);
+    const int m = min(4, n - i);
+    double o[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (k < m) {
+        o[k] = rec_step<REF>(v[k], y1, y2, y3, a.B, a.a1, a.a2, a.a3);
+        y3 = y2;
+        y2 = y1;
+        y1 = o[k];
+      } else {
+        o[k] = 0.0;
+      }
+      v[k] = nx[k];
+    }
+    rec_store4<CONTIG>(p + i * s, s, m, o);
+  }
+  // backwards from the steady state of the last causal sample (y1), the last
+  // group first
+  y2 = y1;
+  y3 = y1;
+  const int top = (n - 1) / 4 * 4;
+  rec_load4<CONTIG>(p + top * s, s, n - top, v);
+  for (int i = top; i >= 0; i -= 4) {
+    if (i >= 4) rec_load4<CONTIG>(p + (i - 4) * s, s, 4, nx);
+    const int m = min(4, n - i);
+    double o[4];
+#pragma unroll
+    for (int k = 3; k >= 0; --k) {
+      if (k < m) {
+        o[k] = rec_step<REF>(v[k], y1, y2, y3, a.B, a.a1, a.a2, a.a3);
+        y3 = y2;
+        y2 = y1;
+        y1 = o[k];
+      } else {
+        o[k] = 0.0;
+      }
+      v[k] = nx[k];
+    }
+    if constexpr (LAST) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (i + k >= w0 && i + k < w1) rec_write(op + (int64_t)(i + k) * os, a.out.dtype, o[k]);
+    } else {
+      rec_store4<CONTIG>(p + i * s, s, m, o);
+    }
+  }
+}
+
+// No axis to filter: the requested region, converted and converted back.
+__global__ void __launch_bounds__(kT) k_rec_copy(RecImage in, RecImage out, int64_t r0, int64_t r1, int64_t r2, int64_t m0,
+                                                  int64_t m1, int64_t m2) {
   const int64_t i = (int64_t)blockIdx.x * kT + threadIdx.x;
   if (i >= m0) return;
   for (int64_t k = blockIdx.z; k < m2; k += gridDim.z)
-    for (int64_t j = blockIdx.y; j < m1; j += gridDim.y) {
-      const int64_t x = r0 + i, y = r1 + j, z = r2 + k;  // absolute
-      const T v = d[((z - g.lo[2]) * g.n[1] + (y - g.lo[1])) * g.n[0] + (x - g.lo[0])];
-      char* p = dst + (x - do0) * dp0 + (y - do1) * dp1 + (z - do2) * dp2;
-      if (OUT == ITKG_U8) *reinterpret_cast<uint8_t*>(p) = out_u8_of((double)v);
-      else *reinterpret_cast<float*>(p) = out_f32(v);
-    }
+    for (int64_t j = blockIdx.y; j < m1; j += gridDim.y)
+      rec_write(out.at + (r0 + i) * out.p[0] + (r1 + j) * out.p[1] + (r2 + k) * out.p[2], out.dtype,
+                rec_read(in.at + (r0 + i) * in.p[0] + (r1 + j) * in.p[1] + (r2 + k) * in.p[2], in.dtype));
 }
 
 // The derivative users (edges.rs:686-950): stencils on the smoothed image `s`
@@ -273,57 +361,68 @@ itkg_status launch_recursive(const itkg_image& in, const itkg_region& largest, c
     g.n[d] = d < D ? (int64_t)largest.size[d] : 1;
     g.lo[d] = d < D ? largest.index[d] : 0;
   }
-  const int64_t total = g.n[0] * g.n[1] * g.n[2];
-  if (total == 0) return ITKG_SUCCESS;
-  double* buf = nullptr;
-  {
-    const itkg_status sa = scratch_alloc(reinterpret_cast<void**>(&buf), (size_t)total * sizeof(double), stream);
-    if (sa != ITKG_SUCCESS) return sa;
-  }
-  int64_t so[3] = {0, 0, 0}, sp[3] = {0, 0, 0}, dof[3] = {0, 0, 0}, dp[3] = {0, 0, 0};
+  if (g.n[0] * g.n[1] * g.n[2] == 0) return ITKG_SUCCESS;
+  if (in.dtype != ITKG_F32 && in.dtype != ITKG_I16 && in.dtype != ITKG_U8 && in.dtype != ITKG_BF16 && in.dtype != ITKG_F16)
+    return set_error(ITKG_ERROR_UNSUPPORTED, "input dtype %d not supported", in.dtype);
+  RecLines a;
+  std::memset(&a, 0, sizeof a);
+  a.g = g;
+  a.pitch = (g.n[0] + 3) / 4 * 4;
+  a.in.at = static_cast<char*>(in.data);
+  a.out.at = static_cast<char*>(out.data);
+  a.in.dtype = in.dtype;
+  a.out.dtype = out.dtype;
+  int axes[3], naxes = 0;  // lines of length <= 1 are left alone (recursive_gaussian.rs:98-100)
   for (int d = 0; d < 3; ++d) {
-    so[d] = d < D ? in.region.index[d] : 0;
-    sp[d] = in.pitch[d];
-    dof[d] = d < D ? out.region.index[d] : 0;
-    dp[d] = out.pitch[d];
-  }
-  const char* src = static_cast<const char*>(in.data);
-  itkg_status st = ITKG_SUCCESS;
-  {  // load the largest region as f64
-    const dim3 gr = grid3(g.n[0], g.n[1], g.n[2]);
-    switch (in.dtype) {
-      case ITKG_F32: k_rec_load<float, double><<<gr, kT, 0, s>>>(src, so[0], so[1], so[2], sp[0], sp[1], sp[2], g, buf); break;
-      case ITKG_I16: k_rec_load<int16_t, double><<<gr, kT, 0, s>>>(src, so[0], so[1], so[2], sp[0], sp[1], sp[2], g, buf); break;
-      case ITKG_U8: k_rec_load<uint8_t, double><<<gr, kT, 0, s>>>(src, so[0], so[1], so[2], sp[0], sp[1], sp[2], g, buf); break;
-      case ITKG_BF16: k_rec_load<__nv_bfloat16, double><<<gr, kT, 0, s>>>(src, so[0], so[1], so[2], sp[0], sp[1], sp[2], g, buf); break;
-      case ITKG_F16: k_rec_load<__half, double><<<gr, kT, 0, s>>>(src, so[0], so[1], so[2], sp[0], sp[1], sp[2], g, buf); break;
-      default: st = set_error(ITKG_ERROR_UNSUPPORTED, "input dtype %d not supported", in.dtype);
+    a.in.p[d] = d < D ? in.pitch[d] : 0;
+    a.out.p[d] = d < D ? out.pitch[d] : 0;
+    if (d < D) {
+      a.in.at += (g.lo[d] - in.region.index[d]) * in.pitch[d];
+      a.out.at += (g.lo[d] - out.region.index[d]) * out.pitch[d];
+      a.lo[d] = requested.index[d] - g.lo[d];
+      a.hi[d] = a.lo[d] + (int64_t)requested.size[d];
+      if ((axis < 0 || d == axis) && g.n[d] > 1) axes[naxes++] = d;
+      if (g.n[d] > INT32_MAX / 2) return set_error(ITKG_ERROR_UNSUPPORTED, "axis %d is too long", d);
+    } else {
+      a.hi[d] = 1;
     }
-    if (st == ITKG_SUCCESS) note_launch("recursive_load");
   }
-  // lines, axis by axis (lines of length <= 1 are left alone, recursive_gaussian.rs:98-100)
-  for (int a = 0; a < D && st == ITKG_SUCCESS; ++a) {
-    if (axis >= 0 && a != axis) continue;
-    if (g.n[a] <= 1) continue;
+  itkg_status st = ITKG_SUCCESS;
+  double* buf = nullptr;
+  if (naxes == 0) {
+    k_rec_copy<<<grid3(a.hi[0] - a.lo[0], a.hi[1] - a.lo[1], a.hi[2] - a.lo[2]), kT, 0, s>>>(
+        a.in, a.out, a.lo[0], a.lo[1], a.lo[2], a.hi[0] - a.lo[0], a.hi[1] - a.lo[1], a.hi[2] - a.lo[2]);
+    note_launch("recursive_copy");
+  } else {
+    st = scratch_alloc(reinterpret_cast<void**>(&buf), (size_t)(a.pitch * g.n[1] * g.n[2]) * sizeof(double), stream);
+    if (st != ITKG_SUCCESS) return st;
+    a.d = buf;
+  }
+  using Fn = void (*)(const RecLines);
+  static const Fn fns[2][2][2][2] = {  // [ref][first][last][axis 0]
+      {{{k_rec_lines<false, false, false, false>, k_rec_lines<false, false, false, true>},
+        {k_rec_lines<false, false, true, false>, k_rec_lines<false, false, true, true>}},
+       {{k_rec_lines<false, true, false, false>, k_rec_lines<false, true, false, true>},
+        {k_rec_lines<false, true, true, false>, k_rec_lines<false, true, true, true>}}},
+      {{{k_rec_lines<true, false, false, false>, k_rec_lines<true, false, false, true>},
+        {k_rec_lines<true, false, true, false>, k_rec_lines<true, false, true, true>}},
+       {{k_rec_lines<true, true, false, false>, k_rec_lines<true, true, false, true>},
+        {k_rec_lines<true, true, true, false>, k_rec_lines<true, true, true, true>}}}};
+  for (int i = 0; i < naxes; ++i) {
+    const int d = axes[i];
     double c[4];
-    yvv_coeffs(sigma / in.spacing[a], c);
-    const unsigned blocks = (unsigned)((total / g.n[a] + kT - 1) / kT);
-    if (ref) k_rec_lines<double, true><<<blocks, kT, 0, s>>>(buf, g, a, c[0], c[1], c[2], c[3]);
-    else k_rec_lines<double, false><<<blocks, kT, 0, s>>>(buf, g, a, c[0], c[1], c[2], c[3]);
+    yvv_coeffs(sigma / in.spacing[d], c);
+    a.axis = d;
+    a.in_step = a.in.p[d];
+    a.out_step = a.out.p[d];
+    a.w0 = (int32_t)a.lo[d], a.w1 = (int32_t)a.hi[d];
+    a.B = c[0], a.a1 = c[1], a.a2 = c[2], a.a3 = c[3];
+    const int64_t lines = g.n[0] * g.n[1] * g.n[2] / g.n[d];
+    const unsigned blocks = (unsigned)((lines + 31) / 32);
+    fns[ref ? 1 : 0][i == 0][i + 1 == naxes][d == 0]<<<blocks, 32, 0, s>>>(a);
     note_launch(ref ? "recursive_lines_f64" : "recursive_lines_f64_fma");
   }
-  if (st == ITKG_SUCCESS) {  // the requested region, converted
-    int64_t r[3] = {0, 0, 0}, m[3] = {1, 1, 1};
-    for (int d = 0; d < D; ++d) r[d] = requested.index[d], m[d] = (int64_t)requested.size[d];
-    const dim3 gr = grid3(m[0], m[1], m[2]);
-    char* dst = static_cast<char*>(out.data);
-    if (out.dtype == ITKG_U8)
-      k_rec_store<double, ITKG_U8><<<gr, kT, 0, s>>>(buf, g, r[0], r[1], r[2], m[0], m[1], m[2], dst, dof[0], dof[1],
-                                                     dof[2], dp[0], dp[1], dp[2]);
-    else
-      k_rec_store<double, ITKG_F32><<<gr, kT, 0, s>>>(buf, g, r[0], r[1], r[2], m[0], m[1], m[2], dst, dof[0], dof[1],
-                                                      dof[2], dp[0], dp[1], dp[2]);
-    note_launch("recursive_store");
+  {
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) st = set_error(ITKG_ERROR_CUDA, "recursive gaussian launch: %s", cudaGetErrorString(e));
   }
