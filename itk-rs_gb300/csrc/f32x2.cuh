@@ -1,8 +1,10 @@
 // Packed two-lane f32 arithmetic (PTX add/mul/fma .f32x2, sm_100+).
-// Reference rounding does not use these: a packed mul.rn / add.rn pair was
-// measured on the GPU to give results that differ from the scalar
-// __fmul_rn / __fadd_rn sequence (in about 70% of the voxels of a 3-D filter),
-// so every reference-rounding tap is scalar.
+// The FP32 pipe does 128 lanes per clock and SM either way (measured 123 - 126,
+// scalar or packed, multiply, add or FMA); packing halves the issue slots.
+// ptxas contracts a packed mul.rn feeding an add.rn into an FMA (they ran at
+// the FMA's rate, and a 3-D filter differed in about 70% of its voxels), so
+// reference rounding never pairs the two: its product is fma2(x, w, -0) with
+// the -0 a kernel argument, which rounds x * w once and cannot be folded.
 #pragma once
 
 #include <cstdint>

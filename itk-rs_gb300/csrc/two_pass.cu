@@ -21,6 +21,7 @@ ZFn z_fn(int r, bool ref, int store, bool ush) {
   switch (store) {
     case kStoreAny: row = ref ? z_row_ref_any() : z_row_fma_any(); break;
     case kStoreF32Quad: row = ref ? z_row_ref_f32q() : z_row_fma_f32q(); break;
+    case kStoreF32Ragged: row = ref ? z_row_ref_f32rag() : z_row_fma_f32rag(); break;
     case kStoreBF16Quad: row = ref ? z_row_ref_bf16q() : z_row_fma_bf16q(); break;
     case kStoreF16Quad: row = ref ? z_row_ref_f16q() : z_row_fma_f16q(); break;
     default: return nullptr;
@@ -194,23 +195,24 @@ itkg_status launch_two_pass(const FusedGeom& g, const float* const w[kMaxDim], v
   if (!fits_i32(nx) || !fits_i32(ny)) return ITKG_ERROR_UNSUPPORTED;
   const int64_t ntx = (nx + twopass::kTileX - 1) / twopass::kTileX;
   const int64_t nty = (ny + e->ty - 1) / e->ty;
-  // one store per quad (16 bytes of f32, 8 bytes of bf16 / f16) when every
-  // quad of the output is full and aligned
+  // one store per quad (16 bytes of f32, 8 bytes of bf16 / f16, 4 of u8) when
+  // the output's quads are aligned, in the ragged variants too for rows that
+  // end in a partial quad (bf16 and f16 ones: the general variant)
   char* const dst0 = static_cast<char*>(g.dst) + (g.req_index[0] - g.dst_origin[0]) * g.dst_pitch[0] +
                      (g.req_index[1] - g.dst_origin[1]) * g.dst_pitch[1];
+  const int osz = dtype_size(g.out_dtype);
+  const int64_t qa = 4 * osz;  // bytes per quad
+  const bool quads = g.dst_pitch[0] == osz && ((uintptr_t)dst0 % qa) == 0 && g.dst_pitch[1] % qa == 0 &&
+                     g.dst_pitch[2] % qa == 0;
   int store = twopass::kStoreAny;
-  if (u8p) {
-    if (g.dst_pitch[0] == 1 && ((uintptr_t)dst0 & 3) == 0 && g.dst_pitch[1] % 4 == 0 && g.dst_pitch[2] % 4 == 0 &&
-        nx % 4 == 0)
-      store = twopass::kStoreU8Quad;
-  } else {
-    const int osz = g.out_dtype == ITKG_F32 ? 4 : (g.out_dtype == ITKG_BF16 || g.out_dtype == ITKG_F16) ? 2 : 0;
-    const int64_t qa = 4 * osz;  // bytes per quad
-    if (osz && g.dst_pitch[0] == osz && ((uintptr_t)dst0 % qa) == 0 && g.dst_pitch[1] % qa == 0 &&
-        g.dst_pitch[2] % qa == 0 && nx % 4 == 0)
-      store = g.out_dtype == ITKG_F32    ? twopass::kStoreF32Quad
-              : g.out_dtype == ITKG_BF16 ? twopass::kStoreBF16Quad
-                                         : twopass::kStoreF16Quad;
+  if (quads && nx % 4 == 0) {
+    if (u8p) store = twopass::kStoreU8Quad;
+    else if (g.out_dtype == ITKG_F32) store = twopass::kStoreF32Quad;
+    else if (g.out_dtype == ITKG_BF16) store = twopass::kStoreBF16Quad;
+    else if (g.out_dtype == ITKG_F16) store = twopass::kStoreF16Quad;
+  } else if (quads) {
+    if (u8p) store = twopass::kStoreU8Ragged;
+    else if (g.out_dtype == ITKG_F32) store = twopass::kStoreF32Ragged;
   }
   const bool vec = store == twopass::kStoreF32Quad;
   // the unsharp store reads the input's quads at the output's positions (the
@@ -254,7 +256,9 @@ itkg_status launch_two_pass(const FusedGeom& g, const float* const w[kMaxDim], v
   xa.wait_limit = wait_limit_cycles();
   int res_xy = 0, res_z = 0;
   const twopass::ZFn zfn =
-      u8p ? (store == twopass::kStoreU8Quad ? twopass::z_row_u8p_u8q() : twopass::z_row_u8p_any())[rz - 1]
+      u8p ? (store == twopass::kStoreU8Quad     ? twopass::z_row_u8p_u8q()
+             : store == twopass::kStoreU8Ragged ? twopass::z_row_u8p_u8rag()
+                                                : twopass::z_row_u8p_any())[rz - 1]
           : twopass::z_fn(rz, ref, store, ush != nullptr);
   const twopass::XYFn xyfn = e->fn[ref ? 1 : 0];
   if (st == ITKG_SUCCESS) st = max_resident_ctas(reinterpret_cast<const void*>(xyfn), e->smem, e->nt, &res_xy);
@@ -265,6 +269,7 @@ itkg_status launch_two_pass(const FusedGeom& g, const float* const w[kMaxDim], v
     return st;
   }
 
+  za.negz = -0.0f;
   xa.t = t;
   xa.t_slice = slice_floats;
   for (int d = 0; d < 3; ++d) {
@@ -325,7 +330,7 @@ itkg_status launch_two_pass(const FusedGeom& g, const float* const w[kMaxDim], v
   za.dst_pitch[0] = g.dst_pitch[0];
   za.dst_pitch[1] = g.dst_pitch[1];
   za.dst_pitch[2] = g.dst_pitch[2];
-  za.vec_store = store;
+  za.quads = quads ? 1 : 0;
   if (ush) {
     za.ush = *ush;
     za.ush_pitch[0] = g.src_pitch[0];

@@ -27,7 +27,7 @@
 // w[k] * v); output j - RZ is complete and stored.  The loop is unrolled over
 // the KZ phases so every ring slot is a compile-time register.
 //
-// Reference rounding: scalar acc = acc + x * w with separate roundings, in
+// Reference rounding: acc = acc + x * w with separate roundings, in
 // ascending tap order from zero, on f32 intermediates -- bit-identical to the
 // reference pass by pass.  FMA rounding: packed fma.rn.f32x2.
 #pragma once
@@ -54,7 +54,8 @@ constexpr int kMaxK = 2 * kMaxR + 1;
 // tile-major: [slice][tile][tile rows][kTileX columns]
 constexpr int kTileX = 32;
 // z-pass store modes (k_z_pass's ST)
-constexpr int kStoreAny = 0, kStoreF32Quad = 1, kStoreBF16Quad = 2, kStoreF16Quad = 3, kStoreU8Quad = 4;
+constexpr int kStoreAny = 0, kStoreF32Quad = 1, kStoreBF16Quad = 2, kStoreF16Quad = 3, kStoreU8Quad = 4,
+              kStoreF32Ragged = 5, kStoreU8Ragged = 6;
 constexpr int kMaxZSplit = 1024;  // z-pass CTAs with a per-CTA unit range
 constexpr int kTileY = 128;  // the tallest tile
 
@@ -102,12 +103,13 @@ struct ZArgs {
   char* dst;               // output voxel (x0, y0, z0)
   int64_t dst_pitch[3];    // bytes
   int32_t out_dtype;
-  int32_t vec_store;       // store mode of the launched variant (kStore*, see k_z_pass)
+  int32_t quads;           // kStoreAny: the output's whole quads are aligned for one store each
   const char* ush_src;     // UnsharpMaskFilter variant: input voxel (x0, y0, z0)
   int64_t ush_pitch[3];    // bytes
   UnsharpConsts ush;
   float wz[kMaxK];
   f2_t wz2[kMaxK];
+  float negz;              // -0 (reference rounding, see tap2_ref)
   int32_t nsplit;          // > 0: CTA b processes units [split[b], split[b + 1]); 0: an even split
   int32_t split[kMaxZSplit + 1];
 };
@@ -202,21 +204,33 @@ __device__ __forceinline__ float ld1(const __half* p) { return __half2float(*p);
 // wrapping add, so a pass's output is the sum of its taps' values mod 256, in
 // any order.  A tap's value is computed in f32: floor(fma(v, c, 0.5)) with a
 // per-tap constant c that the host has checked against the f64 definition for
-// all 256 values of v (an f32 near w; see u8_pixel_tap_consts).  Adding 2^23
-// rounding down leaves floor(.) in the low mantissa bits of 2^23 + floor(.), a
-// bit pattern whose low byte is the tap's value, so the taps' bit patterns are
-// summed as integers and the sum's low byte is the pass's output.
-__device__ __forceinline__ uint32_t u8p_tap(float v, float c) {
-  return __float_as_uint(__fadd_rd(__fmaf_rn(v, c, 0.5f), 8388608.0f));
+// all 256 values of v (an f32 near w; see u8_pixel_tap_consts).  An accumulator
+// holds 2^23 + the sum so far: adding fma(v, c, 0.5) to it rounding down adds
+// the tap's floor, because f32s between 2^23 and 2^24 are the integers (the sum
+// of 25 taps stays below 2^13).  The low byte of its bit pattern is the pass's
+// output.  Two packed instructions per pair of taps; summing the taps' bit
+// patterns as integers took a third one per tap.
+constexpr f2_t kU8pZero = 0x4B0000004B000000ull;  // 2^23 in both lanes
+__device__ __forceinline__ f2_t u8p_tap2(f2_t acc, f2_t v, f2_t c) {
+  f2_t t, r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(t) : "l"(v), "l"(c), "l"(0x3F0000003F000000ull));
+  asm("add.rm.f32x2 %0, %1, %2;" : "=l"(r) : "l"(acc), "l"(t));
+  return r;
 }
-// the low byte of an accumulated sum, as an exact f32 (0 .. 255)
+// the low byte of an accumulator's bit pattern, as an exact f32 (0 .. 255)
 __device__ __forceinline__ float u8p_value(uint32_t acc) {
   return __fsub_rn(__uint_as_float(0x4B000000u | (acc & 255u)), 8388608.0f);
 }
 
+// Reference rounding on two lanes: acc + x * w with both operations rounded.
+// ptxas contracts a packed mul and add into an FMA, so the product is
+// fma(x, w, nz) with nz a kernel argument that holds -0: x * w rounded once,
+// the sign of a zero product kept.
+__device__ __forceinline__ f2_t tap2_ref(f2_t acc, f2_t x, f2_t w, f2_t nz) { return add2(acc, fma2(x, w, nz)); }
+
 // ---------------------------------------------------------------------------
 // xy pass
-// U8P (with REF and u8 input): u8 pixel arithmetic; a.wx / a.wy hold the
+// U8P (with REF and u8 input): u8 pixel arithmetic; the weights are the
 // per-tap constants c, and T holds each y-pass output byte as an f32.
 template <int R, bool REF, typename Tin, bool U8P = false>
 __global__ void __launch_bounds__(288, CfgXY<R, Tin>::MINB)
@@ -291,14 +305,23 @@ __global__ void __launch_bounds__(288, CfgXY<R, Tin>::MINB)
           v[q] = c0 + q > cr ? vr : v[q];
         }
       }
+      if constexpr (U8P) {
+        // the taps' order does not matter: tap pairs as in FMA rounding, the
+        // lanes' sums added (the padding tap's constant 0 adds nothing)
+        f2_t E[WIN / 2];
 #pragma unroll
-      for (int m = 0; m < MX; ++m) {
-        if constexpr (U8P) {
-          uint32_t ia = 0;
+        for (int q = 0; q < WIN / 2; ++q) E[q] = pack2(v[2 * q], v[2 * q + 1]);
 #pragma unroll
-          for (int k = 0; k < K; ++k) ia += u8p_tap(v[m + k + OFF], a.wx[k]);
-          o[m] = u8p_value(ia);
-        } else {
+        for (int m = 0; m < MX; ++m) {
+          const int q0 = m + OFF;
+          f2_t ax = kU8pZero;
+#pragma unroll
+          for (int i = 0; i <= R; ++i) ax = u8p_tap2(ax, E[q0 / 2 + i], (q0 & 1) ? a.wo[i] : a.we[i]);
+          o[m] = u8p_value((uint32_t)ax + (uint32_t)(ax >> 32));
+        }
+      } else {
+#pragma unroll
+        for (int m = 0; m < MX; ++m) {
           float ax = 0.0f;
 #pragma unroll
           for (int k = 0; k < K; ++k) ax = tap<true>(ax, v[m + k + OFF], a.wx[k]);
@@ -411,15 +434,10 @@ __global__ void __launch_bounds__(288, CfgXY<R, Tin>::MINB)
 #pragma unroll
         for (int m = 0; m < MY; ++m) {
           if constexpr (U8P) {
-            uint32_t i0 = 0, i1 = 0;
+            f2_t ay = kU8pZero;
 #pragma unroll
-            for (int k = 0; k < K; ++k) {
-              float v0, v1;
-              unpack2(win[m + k], v0, v1);
-              i0 += u8p_tap(v0, a.wy[k]);
-              i1 += u8p_tap(v1, a.wy[k]);
-            }
-            yv[m] = pack2(u8p_value(i0), u8p_value(i1));
+            for (int k = 0; k < K; ++k) ay = u8p_tap2(ay, win[m + k], a.wy2[k]);
+            yv[m] = pack2(u8p_value((uint32_t)ay), u8p_value((uint32_t)(ay >> 32)));
           } else if constexpr (REF) {
             float y0 = 0.0f, y1 = 0.0f;
 #pragma unroll
@@ -498,27 +516,43 @@ timeout:
 
 // ---------------------------------------------------------------------------
 // z pass
-// ST: how a completed quad is stored.  kStoreAny: element by element, any
-// output type and width.  kStoreF32Quad: one 16-byte store (f32 output whose
-// rows allow it and whose width is a multiple of 4, every quad full).
-// kStoreBF16Quad / kStoreF16Quad: the same for bf16 / f16 output, one 8-byte
-// store of the four rounded values.  kStoreU8Quad (U8P only): one 4-byte store.
-// U8P (with REF): u8 pixel arithmetic over T's bytes (see u8p_tap), a.wz
-// holding the per-tap constants; the output is u8.
+// ST: how a completed quad is stored.  kStoreF32Quad: one 16-byte store (f32
+// output whose rows allow it and whose width is a multiple of 4, every quad
+// full).  kStoreBF16Quad / kStoreF16Quad: the same for bf16 / f16 output, one
+// 8-byte store of the four rounded values.  kStoreU8Quad (U8P only): one 4-byte
+// store.  kStoreF32Ragged / kStoreU8Ragged: the same for rows whose last quad
+// is partial, which goes element by element.  kStoreAny: any output; with
+// a.quads (rows that allow it) one store per whole quad.  197 x 233 x 189,
+// reference rounding, RZ = 5, the call: 57.9 us element by element, 54.0 us
+// with the choice by type at run time, 47.4 us ragged; the partial quad's code
+// costs a full-width volume 1 %, hence the two variants.
+// U8P (with REF): u8 pixel arithmetic over T's bytes (see u8p_tap2), the
+// weights being the per-tap constants; the output is u8.
 // USH (with kStoreF32Quad): store UnsharpMaskFilter's
 // point-wise step of the input voxel and the blur instead of the blur --
 // unsharp_cheap_f32 in FMA rounding, the exact f32 test (unsharp_quad_exact,
 // one out-of-line copy) in reference rounding; the input quads travel in a
 // second cp.async ring beside the T quads (the input quad of output z rides
 // with T slice z + RZ).
+// Reference rounding: scalar products and sums up to RZ = 6, packed ones from
+// RZ = 7 on.  The FP32 pipe's time is the same; with two CTAs per SM the scalar
+// form's longer run of independent chains is ahead (192^3, RZ = 5: 13.6 against
+// 14.3 us), with one CTA the packed form's fewer instructions are (RZ = 12: 40
+// against 66 us).  Two CTAs while the accumulators fit 128 registers: up to
+// RZ = 8, in reference rounding and u8 pixel arithmetic up to 6 (RZ = 8 spilled:
+// 23.6 against 18.8 us with one CTA).
 template <int RZ, bool REF, int ST, bool USH = false, bool U8P = false>
-__global__ void __launch_bounds__(256, RZ <= 8 ? 2 : 1) k_z_pass(const __grid_constant__ ZArgs a) {
+__global__ void __launch_bounds__(256, RZ <= (REF ? 6 : 8) ? 2 : 1) k_z_pass(const __grid_constant__ ZArgs a) {
   static_assert(!USH || ST == kStoreF32Quad, "the unsharp variant stores whole f32 quads");
-  static_assert(!U8P || (REF && !USH && (ST == kStoreAny || ST == kStoreU8Quad)), "u8 pixel arithmetic stores u8");
-  static_assert(ST != kStoreU8Quad || U8P, "the u8 quad store is the u8 pixel arithmetic's");
+  static_assert(!U8P || (REF && !USH && (ST == kStoreAny || ST == kStoreU8Quad || ST == kStoreU8Ragged)),
+                "u8 pixel arithmetic stores u8");
+  static_assert((ST != kStoreU8Quad && ST != kStoreU8Ragged) || U8P, "the u8 quad store is the u8 pixel arithmetic's");
   using C = CfgZ<RZ>;
   constexpr int KZ = C::KZ, S = C::S, NT = C::NT;
   static_assert(C::QPT == 1, "one quad per thread");
+  constexpr f2_t kZero = U8P ? kU8pZero : 0ull;
+  constexpr bool kPacked = RZ >= 7;
+  [[maybe_unused]] const f2_t nz = pack2(a.negz, a.negz);
   extern __shared__ __align__(16) float4 zring[];  // [S][NT], then (USH) the input ring [S][NT]
   const int tid = threadIdx.x;
   const int64_t u_begin = a.nsplit > 0 ? (int64_t)a.split[blockIdx.x] : a.units * blockIdx.x / gridDim.x;
@@ -571,8 +605,10 @@ __global__ void __launch_bounds__(256, RZ <= 8 ? 2 : 1) k_z_pass(const __grid_co
 #pragma unroll
     for (int m = 0; m < 2; ++m)
 #pragma unroll
-      for (int k = 0; k < KZ; ++k) acc[m][k] = 0ull;
+      for (int k = 0; k < KZ; ++k) acc[m][k] = kZero;
     const int ncols = min(4, a.nx - cx);
+    // whether this thread's quads go in one store (run-time choice)
+    const bool whole = (ST == kStoreAny ? a.quads != 0 : true) && ncols == 4;
     char* dz = a.dst + (int64_t)cx * a.dst_pitch[0] + (int64_t)cy * a.dst_pitch[1] +
                (int64_t)(z0 - a.z0) * a.dst_pitch[2];
     // One slice at phase p (a constant once the callers' loops are unrolled):
@@ -591,16 +627,16 @@ __global__ void __launch_bounds__(256, RZ <= 8 ? 2 : 1) k_z_pass(const __grid_co
 #pragma unroll
         for (int m = 0; m < 2; ++m) {
           if constexpr (U8P) {
-            float v0, v1;
-            unpack2(v[m], v0, v1);
-            const uint32_t a0 = (uint32_t)acc[m][slot] + u8p_tap(v0, a.wz[k]);
-            const uint32_t a1 = (uint32_t)(acc[m][slot] >> 32) + u8p_tap(v1, a.wz[k]);
-            acc[m][slot] = ((f2_t)a1 << 32) | a0;
+            acc[m][slot] = u8p_tap2(acc[m][slot], v[m], a.wz2[k]);
           } else if constexpr (REF) {
-            float a0, a1, v0, v1;
-            unpack2(acc[m][slot], a0, a1);
-            unpack2(v[m], v0, v1);
-            acc[m][slot] = pack2(__fadd_rn(a0, __fmul_rn(v0, a.wz[k])), __fadd_rn(a1, __fmul_rn(v1, a.wz[k])));
+            if constexpr (kPacked) {
+              acc[m][slot] = tap2_ref(acc[m][slot], v[m], a.wz2[k], nz);
+            } else {
+              float a0, a1, v0, v1;
+              unpack2(acc[m][slot], a0, a1);
+              unpack2(v[m], v0, v1);
+              acc[m][slot] = pack2(tap<true>(a0, v0, a.wz[k]), tap<true>(a1, v1, a.wz[k]));
+            }
           } else if (k == 0) {  // first contribution to output j + RZ: its slot was popped
             acc[m][slot] = mul2(v[m], a.wz2[0]);
           } else {
@@ -611,13 +647,13 @@ __global__ void __launch_bounds__(256, RZ <= 8 ? 2 : 1) k_z_pass(const __grid_co
       const int D = (p + 1) % KZ;
       const f2_t d0 = acc[0][D], d1 = acc[1][D];
       if constexpr (REF) {  // reference rounding adds the first product to zero
-        acc[0][D] = 0ull;
-        acc[1][D] = 0ull;
+        acc[0][D] = kZero;
+        acc[1][D] = kZero;
       }
       if (!store) return;
       float o[4];
       if constexpr (U8P) {
-        if constexpr (ST == kStoreU8Quad) {
+        if (ST == kStoreU8Quad || whole) {
           __stcs(reinterpret_cast<unsigned int*>(dz), (uint32_t)(d0 & 255u) | (uint32_t)((d0 >> 24) & 0xFF00u) |
                                                           (uint32_t)((d1 & 255u) << 16) | (uint32_t)((d1 >> 8) & 0xFF000000u));
           dz += a.dst_pitch[2];
@@ -638,9 +674,9 @@ __global__ void __launch_bounds__(256, RZ <= 8 ? 2 : 1) k_z_pass(const __grid_co
           __stcs(reinterpret_cast<float4*>(dz),
                  make_float4(unsharp_cheap_f32(og.x, o[0], a.ush), unsharp_cheap_f32(og.y, o[1], a.ush),
                              unsharp_cheap_f32(og.z, o[2], a.ush), unsharp_cheap_f32(og.w, o[3], a.ush)));
-      } else if constexpr (ST == kStoreF32Quad) {
+      } else if (ST == kStoreF32Quad || (ST == kStoreF32Ragged && whole)) {
         __stcs(reinterpret_cast<float4*>(dz), make_float4(o[0], o[1], o[2], o[3]));
-      } else if constexpr (ST == kStoreBF16Quad || ST == kStoreF16Quad) {
+      } else if (ST == kStoreBF16Quad || ST == kStoreF16Quad) {
         uint32_t h[4];
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
@@ -648,12 +684,32 @@ __global__ void __launch_bounds__(256, RZ <= 8 ? 2 : 1) k_z_pass(const __grid_co
           else h[c] = __half_as_ushort(from_f32<__half>(o[c]));
         }
         __stcs(reinterpret_cast<uint2*>(dz), make_uint2(h[0] | (h[1] << 16), h[2] | (h[3] << 16)));
+      } else if (ST == kStoreAny && whole) {
+        switch (a.out_dtype) {
+          case ITKG_F32: __stcs(reinterpret_cast<float4*>(dz), make_float4(o[0], o[1], o[2], o[3])); break;
+          case ITKG_BF16:
+          case ITKG_F16: {
+            uint32_t h[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+              h[c] = a.out_dtype == ITKG_BF16 ? __bfloat16_as_ushort(from_f32<__nv_bfloat16>(o[c]))
+                                              : __half_as_ushort(from_f32<__half>(o[c]));
+            __stcs(reinterpret_cast<uint2*>(dz), make_uint2(h[0] | (h[1] << 16), h[2] | (h[3] << 16)));
+            break;
+          }
+          default: {
+            uint32_t h = 0;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) h |= (uint32_t)from_f32<uint8_t>(o[c]) << (8 * c);
+            __stcs(reinterpret_cast<uint32_t*>(dz), h);
+          }
+        }
       } else {
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           if (c >= ncols) break;
           char* const dp = dz + c * a.dst_pitch[0];
-          switch (a.out_dtype) {
+          switch (ST == kStoreF32Ragged ? ITKG_F32 : ST == kStoreU8Ragged ? ITKG_U8 : a.out_dtype) {
             case ITKG_F32: *reinterpret_cast<float*>(dp) = o[c]; break;
             case ITKG_BF16: *reinterpret_cast<__nv_bfloat16*>(dp) = from_f32<__nv_bfloat16>(o[c]); break;
             case ITKG_F16: *reinterpret_cast<__half*>(dp) = from_f32<__half>(o[c]); break;
@@ -724,6 +780,9 @@ const ZFn* z_row_ref_f16q();    //                          REF true, kStoreF16Q
 const XYEntry* xy_entries_u8p(int* n);
 const ZFn* z_row_u8p_any();
 const ZFn* z_row_u8p_u8q();
+const ZFn* z_row_u8p_u8rag();
+const ZFn* z_row_fma_f32rag();  // two_pass_zrag.cu: REF false, kStoreF32Ragged
+const ZFn* z_row_ref_f32rag();  //                   REF true, kStoreF32Ragged
 ZFn z_ush_fn(int r, bool ref);  // two_pass_ush.cu
 
 #define ITKG_Z_ROW(REF, ST)                                                                             \

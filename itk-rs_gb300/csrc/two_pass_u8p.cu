@@ -39,5 +39,9 @@ const ZFn* z_row_u8p_u8q() {
   static const ZFn row[kMaxR] = ITKG_Z_U8P_ROW(kStoreU8Quad);
   return row;
 }
+const ZFn* z_row_u8p_u8rag() {
+  static const ZFn row[kMaxR] = ITKG_Z_U8P_ROW(kStoreU8Ragged);
+  return row;
+}
 }  // namespace twopass
 }  // namespace itkg
