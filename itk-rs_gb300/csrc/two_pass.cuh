@@ -669,7 +669,8 @@ __global__ void __launch_bounds__(256, RZ <= (REF ? 6 : 8) ? 2 : 1) k_z_pass(con
       }
       if constexpr (USH) {
         if constexpr (REF)
-          __stcs(reinterpret_cast<float4*>(dz), unsharp_quad_exact(og, o[0], o[1], o[2], o[3], a.ush));
+          __stcs(reinterpret_cast<float4*>(dz), a.ush.a_exact ? unsharp_quad_front(og, o[0], o[1], o[2], o[3], a.ush)
+                                                              : unsharp_quad_exact(og, o[0], o[1], o[2], o[3], a.ush));
         else
           __stcs(reinterpret_cast<float4*>(dz),
                  make_float4(unsharp_cheap_f32(og.x, o[0], a.ush), unsharp_cheap_f32(og.y, o[1], a.ush),

@@ -18,6 +18,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 
 #include "internal.hpp"
 #include "unsharp.cuh"
@@ -57,9 +58,11 @@ __global__ void __launch_bounds__(kT) k_unsharp(const char* in, int64_t ip0, int
 }
 
 
-// Scalar f32 rows of 16-byte aligned quads (x pitch 4, width a multiple of 4,
-// 16-byte aligned rows): thread i of the grid takes quads i, i + grid, ... of
-// the rows x quads space, streaming loads and stores.  I: the index type
+// Scalar f32 rows of 16-byte aligned quads (x pitch 4, 16-byte aligned rows; the
+// last quad of a row may be ragged): thread i of the grid takes quads i, i +
+// grid, ... of the rows x quads space, streaming loads and stores.  The blur may
+// be the output image itself: a thread reads its quads before it writes them,
+// and a deferred voxel keeps its blur until k_unsharp_deferred replaces it.  I: the index type
 // (32-bit when the voxel count allows, for cheaper divisions).
 //
 // Voxels the f32 test cannot decide (a few in a thousand on smooth data) are
@@ -67,7 +70,9 @@ __global__ void __launch_bounds__(kT) k_unsharp(const char* in, int64_t ip0, int
 // block appends (quad index * 4 + lane) to its own segment of `defer`
 // (kDeferCap entries; its count in defer_n[block]) and k_unsharp_deferred
 // finishes them afterwards, a handful of f64 sequences per block.  Entries
-// past the segment's capacity are computed in place.
+// past the segment's capacity are computed in place, and so are all with
+// defer NULL (FMA rounding and amounts that are f32: the f32 rules leave next
+// to none open).
 constexpr int kQT = 256;
 constexpr int kDeferCap = 2048;
 
@@ -80,14 +85,23 @@ __device__ __forceinline__ void quad_addr(I i, I nq, I m1, int64_t p1, int64_t p
   off = (int64_t)y * p1 + (int64_t)z * p2;
 }
 
+// The first n (< 4) floats of a quad, zeros after them.
+__device__ __forceinline__ float4 load_ragged(const float* p, int n) {
+  return make_float4(p[0], n > 1 ? p[1] : 0.0f, n > 2 ? p[2] : 0.0f, 0.0f);
+}
+
 template <typename I>
 __global__ void __launch_bounds__(kQT) k_unsharp_quads(const char* in, int64_t ip1, int64_t ip2, const char* blur,
                                                         int64_t bp1, int64_t bp2, char* out, int64_t op1, int64_t op2,
-                                                        I nq, I m1, I total, const UnsharpConsts k, I* defer,
+                                                        I nq, I m0, I m1, I total, const UnsharpConsts k, I* defer,
                                                         uint32_t* defer_n) {
   __shared__ uint32_t n_def;
   if (threadIdx.x == 0) n_def = 0;
   __syncthreads();
+  // a programmatic dependent of the blur's last kernel, and the next call's
+  // first kernel may be one of this: each waits before it touches memory
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
   I* const seg = defer + (size_t)blockIdx.x * kDeferCap;
   // two quads per step (i and i + stride), their loads issued together
   const I stride = (I)gridDim.x * kQT;
@@ -96,6 +110,7 @@ __global__ void __launch_bounds__(kQT) k_unsharp_quads(const char* in, int64_t i
     int64_t ooff[2];
     I qxs[2];
     bool live[2];
+    int ncols[2];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       const I i = i0 + (I)h * stride;
@@ -107,8 +122,16 @@ __global__ void __launch_bounds__(kQT) k_unsharp_quads(const char* in, int64_t i
       const I y = row - z * m1;
       qxs[h] = qx;
       ooff[h] = (int64_t)y * op1 + (int64_t)z * op2;
-      o[h] = __ldcs(reinterpret_cast<const float4*>(in + (int64_t)y * ip1 + (int64_t)z * ip2) + qx);
-      b[h] = __ldcs(reinterpret_cast<const float4*>(blur + (int64_t)y * bp1 + (int64_t)z * bp2) + qx);
+      const float4* const oq = reinterpret_cast<const float4*>(in + (int64_t)y * ip1 + (int64_t)z * ip2) + qx;
+      const float4* const bq = reinterpret_cast<const float4*>(blur + (int64_t)y * bp1 + (int64_t)z * bp2) + qx;
+      ncols[h] = (int)min((I)4, m0 - 4 * qx);
+      if (ncols[h] == 4) {
+        o[h] = __ldcs(oq);
+        b[h] = __ldcs(bq);
+      } else {
+        o[h] = load_ragged(reinterpret_cast<const float*>(oq), ncols[h]);
+        b[h] = load_ragged(reinterpret_cast<const float*>(bq), ncols[h]);
+      }
     }
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
@@ -120,19 +143,25 @@ __global__ void __launch_bounds__(kQT) k_unsharp_quads(const char* in, int64_t i
       for (int c = 0; c < 4; ++c) {
         if (k.cheap) {
           r[c] = unsharp_cheap_f32(ov[c], bv[c], k);
-        } else if (!unsharp_fast_f32(ov[c], bv[c], k, r[c])) {
-          const uint32_t slot = atomicAdd(&n_def, 1u);
+        } else if (!(k.a_exact && unsharp_front_f32(ov[c], bv[c], k, r[c])) && !unsharp_fast_f32(ov[c], bv[c], k, r[c])) {
+          const uint32_t slot = defer ? atomicAdd(&n_def, 1u) : kDeferCap;
           if (slot < kDeferCap) {
             seg[slot] = i * 4 + (I)c;
-            r[c] = ov[c];  // overwritten by k_unsharp_deferred
+            r[c] = bv[c];  // replaced by k_unsharp_deferred
           } else {
             r[c] = __double2float_rn(unsharp_f64((double)ov[c], (double)bv[c], k.amount, k.threshold));
           }
         }
       }
-      __stcs(reinterpret_cast<float4*>(out + ooff[h]) + qxs[h], make_float4(r[0], r[1], r[2], r[3]));
+      float4* const dq = reinterpret_cast<float4*>(out + ooff[h]) + qxs[h];
+      if (ncols[h] == 4) {
+        __stcs(dq, make_float4(r[0], r[1], r[2], r[3]));
+      } else {
+        for (int c = 0; c < ncols[h]; ++c) reinterpret_cast<float*>(dq)[c] = r[c];
+      }
     }
   }
+  if (!defer) return;
   __syncthreads();
   if (threadIdx.x == 0) defer_n[blockIdx.x] = min(n_def, (uint32_t)kDeferCap);
 }
@@ -190,15 +219,34 @@ itkg_status launch_quads(const char* ic, const int64_t* ip, const char* bc, cons
                          const int64_t* op, const int64_t* m, uint64_t total, unsigned blocks, const UnsharpConsts& k,
                          cudaStream_t s) {
   void* scratch = nullptr;
-  const size_t list_bytes = (size_t)blocks * kDeferCap * sizeof(I);
-  itkg_status st = scratch_alloc(&scratch, list_bytes + (size_t)blocks * sizeof(uint32_t), s);
-  if (st != ITKG_SUCCESS) return st;
-  I* const defer = static_cast<I*>(scratch);
-  uint32_t* const defer_n = reinterpret_cast<uint32_t*>(static_cast<char*>(scratch) + list_bytes);
-  k_unsharp_quads<I><<<blocks, kQT, 0, s>>>(ic, ip[1], ip[2], bc, bp[1], bp[2], oc, op[1], op[2], (I)(m[0] / 4),
-                                            (I)m[1], (I)total, k, defer, defer_n);
+  I* defer = nullptr;
+  uint32_t* defer_n = nullptr;
+  if (!k.cheap && !k.a_exact) {
+    const size_t list_bytes = (size_t)blocks * kDeferCap * sizeof(I);
+    const itkg_status st = scratch_alloc(&scratch, list_bytes + (size_t)blocks * sizeof(uint32_t), s);
+    if (st != ITKG_SUCCESS) return st;
+    defer = static_cast<I*>(scratch);
+    defer_n = reinterpret_cast<uint32_t*>(static_cast<char*>(scratch) + list_bytes);
+  }
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg;
+  std::memset(&cfg, 0, sizeof cfg);
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(kQT);
+  cfg.stream = s;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, k_unsharp_quads<I>, ic, ip[1], ip[2], bc, bp[1], bp[2], oc, op[1],
+                                           op[2], (I)((m[0] + 3) / 4), (I)m[0], (I)m[1], (I)total, k, defer, defer_n);
   note_launch("unsharp");
-  k_unsharp_deferred<I><<<blocks, kQT, 0, s>>>(ic, ip[1], ip[2], bc, bp[1], bp[2], oc, op[1], op[2], (I)(m[0] / 4),
+  if (e != cudaSuccess) {
+    scratch_free(scratch, s);
+    return set_error(ITKG_ERROR_CUDA, "unsharp launch: %s", cudaGetErrorString(e));
+  }
+  if (!defer) return ITKG_SUCCESS;
+  k_unsharp_deferred<I><<<blocks, kQT, 0, s>>>(ic, ip[1], ip[2], bc, bp[1], bp[2], oc, op[1], op[2], (I)((m[0] + 3) / 4),
                                                (I)m[1], k, defer, defer_n);
   note_launch("unsharp_deferred");
   scratch_free(scratch, s);
@@ -260,14 +308,14 @@ itkg_status launch_unsharp(int dtype, int comps, const void* in, const int64_t* 
   auto a16 = [](const void* p, int64_t p1, int64_t p2) {
     return ((uintptr_t)p % 16) == 0 && p1 % 16 == 0 && p2 % 16 == 0;
   };
-  const bool quads = dtype == ITKG_F32 && k.fast && comps == 1 && ip[0] == 4 && bp[0] == 4 && op[0] == 4 && m[0] % 4 == 0 &&
-                     m[0] / 4 <= UINT32_MAX && m[1] <= UINT32_MAX && a16(in, ip[1], ip[2]) &&
+  const bool quads = dtype == ITKG_F32 && k.fast && comps == 1 && ip[0] == 4 && bp[0] == 4 && op[0] == 4 &&
+                     m[0] <= INT32_MAX && m[1] <= UINT32_MAX && a16(in, ip[1], ip[2]) &&
                      a16(blur, bp[1], bp[2]) && a16(out, op[1], op[2]);
   if (quads) {
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const uint64_t total = (uint64_t)(m[0] / 4) * (uint64_t)m[1] * (uint64_t)m[2];
+    const uint64_t total = (uint64_t)((m[0] + 3) / 4) * (uint64_t)m[1] * (uint64_t)m[2];
     // one full wave of resident blocks (each thread takes two quads per step)
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_unsharp_quads<uint32_t>, kQT, 0);
