@@ -36,6 +36,7 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <cstring>
 
 #include "f32x2.cuh"
 #include "internal.hpp"
@@ -103,6 +104,14 @@ __device__ __forceinline__ void walk(const f2_t* w2, int R, f2_t nz, f2_t (&acc)
   }
 }
 
+// The passes are programmatic dependents of each other: the next one's blocks
+// may be scheduled as this one's retire (they wait here for it to complete
+// before they touch memory), which hides its launch.
+__device__ __forceinline__ void pdl_begin() {
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+}
+
 struct LineTaps2 {
   f2_t w2[kMaxParamTaps];  // tap k in both lanes
 };
@@ -122,6 +131,7 @@ template <typename Tout, bool REF, bool FULL>
 __global__ void __launch_bounds__(32 * kMaxWarps, 2) k_lines_yz(const __grid_constant__ LinesArgs p,
                                                                 const __grid_constant__ LineTaps2 W) {
   const AxisArgs& a = p.a;
+  pdl_begin();
   const int md = a.axis, od = 3 - md;
   const int64_t rowlen = a.out_size[0] * a.comps;
   const int64_t strip = (int64_t)blockIdx.x * kStrip;
@@ -178,6 +188,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 2) k_lines_x(const __grid_cons
                                                                const __grid_constant__ LineTaps2 W) {
   extern __shared__ float tile[];  // [x position][kRowPitch]
   const AxisArgs& a = p.a;
+  pdl_begin();
   const int warp = threadIdx.y, lane = threadIdx.x, nw = blockDim.y;
   const int64_t nlines = a.out_size[1] * a.out_size[2] * a.comps;
   const int64_t groups = (nlines + kStrip - 1) / kStrip;
@@ -335,9 +346,20 @@ itkg_status launch_conv_lines(const AxisArgs& a, const float* w, int in_dtype, i
   // against 8.4 us) and as fast along y; 97 x 61 x 73 has 140 blocks: 12.7
   // against 8.8 us.
   if (f32 && a.radius <= kMaxSmallRadius && (uint64_t)grid.x * grid.y * grid.z < 128) return ITKG_ERROR_UNSUPPORTED;
-  fn<<<grid, block, smem, s>>>(p, W);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg;
+  std::memset(&cfg, 0, sizeof cfg);
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, fn, p, W);
   note_launch(ref ? "conv_lines_f32_ref" : "conv_lines_f32_fma");
-  const cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return set_error(ITKG_ERROR_CUDA, "conv_lines launch: %s", cudaGetErrorString(e));
   return ITKG_SUCCESS;
 }
