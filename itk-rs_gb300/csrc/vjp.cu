@@ -17,6 +17,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cstring>
 
 #include "internal.hpp"
 #include "pixel.cuh"
@@ -426,6 +427,7 @@ __global__ void __launch_bounds__(kThreads) k_sqerr_q(const float4* __restrict__
 // Fixed-order final sum of the partials (deterministic).
 __global__ void k_sum_partials(const double* partials, int n, double* out, int accumulate) {
   __shared__ double red[kThreads];
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");  // (launched as a programmatic dependent by launch_sum_partials)
   double s = 0.0;
   for (int i = threadIdx.x; i < n; i += kThreads) s += partials[i];
   red[threadIdx.x] = s;
@@ -531,8 +533,18 @@ itkg_status launch_sqerr(const float* y, const float* dy, const DotArgs& t, floa
 
 itkg_status launch_sum_partials(const double* partials, int n, double* out, bool accumulate,
                                 void* stream) {
-  k_sum_partials<<<1, kThreads, 0, static_cast<cudaStream_t>(stream)>>>(partials, n, out,
-                                                                        accumulate ? 1 : 0);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg;
+  std::memset(&cfg, 0, sizeof cfg);
+  cfg.gridDim = dim3(1);
+  cfg.blockDim = dim3(kThreads);
+  cfg.stream = static_cast<cudaStream_t>(stream);
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, k_sum_partials, partials, n, out, accumulate ? 1 : 0);
+  if (e != cudaSuccess) return set_error(ITKG_ERROR_CUDA, "sum_partials_f64 launch: %s", cudaGetErrorString(e));
   return launched("sum_partials_f64");
 }
 

@@ -39,7 +39,28 @@ const Entry* find(int r) {
 }
 
 size_t z_smem(int r) { return (size_t)(2 * r + 1) * 256 * 16; }
-size_t z2_smem(int r) { return (size_t)(2 * r + 1) * 256 * 8; }
+size_t z2_smem(int r) { return (size_t)(2 * r + 1) * kZ2Threads * 8; }
+
+// fn(args...) as a programmatic dependent of the stream's previous kernel
+template <typename F, typename... A>
+itkg_status launch_dependent(const char* name, F fn, int64_t grid, int threads, size_t smem, cudaStream_t s,
+                             const A&... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg;
+  std::memset(&cfg, 0, sizeof cfg);
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaError_t err = cudaLaunchKernelEx(&cfg, fn, args...);
+  note_launch(name);
+  if (err == cudaSuccess) err = cudaGetLastError();
+  return err == cudaSuccess ? ITKG_SUCCESS : set_error(ITKG_ERROR_CUDA, "%s launch: %s", name, cudaGetErrorString(err));
+}
 
 bool aligned16(const itkg_image& im) {
   return ((uintptr_t)im.data & 15) == 0 && im.pitch[0] == 4 && (im.pitch[1] & 15) == 0 && (im.pitch[2] & 15) == 0;
@@ -118,26 +139,22 @@ itkg_status launch_vjp_two_pass(const VjpTwoPass& v, void* stream, bool dry_run)
     vjp2::prefix(v.dw[2], RZ, za.pzd);
     za.out2 = static_cast<char*>(pu2);
     za.npx = (int32_t)((nx + 1) / 2);
-    za.units = ((int64_t)za.npx * ny + 255) / 256 * nz;
+    const int64_t qb = ((int64_t)za.npx * ny + vjp2::kZ2Threads - 1) / vjp2::kZ2Threads;
+    za.units = qb * nz;
     if (st == ITKG_SUCCESS)
-      st = max_resident_ctas(reinterpret_cast<const void*>(ez->z2), vjp2::z2_smem(RZ), 256, &res_z);
+      st = max_resident_ctas(reinterpret_cast<const void*>(ez->z2), vjp2::z2_smem(RZ), vjp2::kZ2Threads, &res_z);
     if (st == ITKG_SUCCESS) {
-      const int64_t g = std::min<int64_t>(za.units, res_z);
-      ez->z2<<<(unsigned)g, 256, vjp2::z2_smem(RZ), s>>>(za);
-      note_launch("z_adjoint2_f32");
-      const cudaError_t err = cudaGetLastError();
-      if (err != cudaSuccess) st = set_error(ITKG_ERROR_CUDA, "z adjoint launch: %s", cudaGetErrorString(err));
+      int64_t g = std::min<int64_t>(za.units, res_z);
+      za.nsplit = z_split(qb, nz, RZ, std::min<int64_t>(g, twopass::kMaxZSplit), za.split);
+      if (za.nsplit > 0) g = za.nsplit;
+      st = vjp2::launch_dependent("z_adjoint2_f32", ez->z2, g, vjp2::kZ2Threads, vjp2::z2_smem(RZ), s, za);
     }
   } else {
     if (st == ITKG_SUCCESS)
       st = max_resident_ctas(reinterpret_cast<const void*>(ez->z), vjp2::z_smem(RZ), 256, &res_z);
-    if (st == ITKG_SUCCESS) {
-      const int64_t g = std::min<int64_t>(za.units, res_z);
-      ez->z<<<(unsigned)g, 256, vjp2::z_smem(RZ), s>>>(za);
-      note_launch("z_adjoint_f32");
-      const cudaError_t err = cudaGetLastError();
-      if (err != cudaSuccess) st = set_error(ITKG_ERROR_CUDA, "z adjoint launch: %s", cudaGetErrorString(err));
-    }
+    if (st == ITKG_SUCCESS)
+      st = vjp2::launch_dependent("z_adjoint_f32", ez->z, std::min<int64_t>(za.units, res_z), 256, vjp2::z_smem(RZ), s,
+                                  za);
   }
 
   // x-y kernels
@@ -149,9 +166,8 @@ itkg_status launch_vjp_two_pass(const VjpTwoPass& v, void* stream, bool dry_run)
     xa.hi[d] = (int32_t)(x.region.index[d] + (int64_t)x.region.size[d] - 1);
   }
   xa.ntx = (int32_t)((nx + e->tx - 1) / e->tx);
-  const int64_t nty = (ny + e->ty - 1) / e->ty;
   xa.ns = (int32_t)nz;
-  xa.units = (int64_t)xa.ntx * nty * nz;
+  xa.units = (int64_t)xa.ntx * ((ny + e->ty - 1) / e->ty) * nz;
   vjp2::tap_pairs(v.w[0], R, xa.we, xa.wo);
   vjp2::tap_pairs(v.dw[0], R, xa.dwe, xa.dwo);
   for (int k = 0; k < 2 * R + 1; ++k) xa.wy2[k] = splat2_host(v.w[1][k]), xa.dwy2[k] = splat2_host(v.dw[1][k]);
@@ -181,6 +197,7 @@ itkg_status launch_vjp_two_pass(const VjpTwoPass& v, void* stream, bool dry_run)
       xa.out = static_cast<char*>(v.xbar->data);
       for (int d = 0; d < 3; ++d) xa.out_pitch[d] = v.xbar->pitch[d];
       xa.accumulate = v.acc_x ? 1 : 0;
+      xa.out_pair = ((uintptr_t)v.xbar->data & 7) == 0 && v.xbar->pitch[1] % 8 == 0 && v.xbar->pitch[2] % 8 == 0;
     } else {
       xa.u = static_cast<const char*>(pu);
       xa.u2 = static_cast<const char*>(pu2);
@@ -189,13 +206,9 @@ itkg_status launch_vjp_two_pass(const VjpTwoPass& v, void* stream, bool dry_run)
       if (st != ITKG_SUCCESS) break;
       xa.partials = static_cast<double*>(ppart);
     }
-    e->xy[mode]<<<(unsigned)grid, 256, e->xy_smem[mode], s>>>(map, xa);
-    note_launch(mode == vjp2::kAdjoint ? "xy_adjoint_f32" : "xy_dual_dot_f32");
-    const cudaError_t err = cudaGetLastError();
-    if (err != cudaSuccess) {
-      st = set_error(ITKG_ERROR_CUDA, "x-y VJP launch: %s", cudaGetErrorString(err));
-      break;
-    }
+    st = vjp2::launch_dependent(mode == vjp2::kAdjoint ? "xy_adjoint_f32" : "xy_dual_dot_f32", e->xy[mode], grid,
+                                256, e->xy_smem[mode], s, map, xa);
+    if (st != ITKG_SUCCESS) break;
     if (mode == vjp2::kDualDot)
       st = launch_sum_partials(xa.partials, (int)grid, v.sigma_out, v.acc_sigma, stream);
   }

@@ -46,7 +46,7 @@ struct XYVArgs {
   char* out;
   int64_t out_pitch[3];
   int32_t accumulate;
-  int32_t pad_;
+  int32_t out_pair;      // xbar's rows allow 8-byte accesses to column pairs
   // dual-dot mode: U (dotted with the derivative) and U' (with the value),
   // f32 with byte pitches; one f64 partial sum per CTA
   const char* u;
@@ -73,9 +73,10 @@ struct ZAArgs {
   // k_z_adj2: the second output (U' = dGz^T ybar) and its weights
   char* out2;
   int32_t npx;             // column pairs per row
-  int32_t pad2_;
+  int32_t nsplit;          // > 0: CTA b processes units [split[b], split[b + 1]); 0: an even split
   f2_t wz2d[kMaxK];
   float pzd[kMaxR + 1];
+  int32_t split[twopass::kMaxZSplit + 1];
 };
 
 template <int R, int MODE>
@@ -104,6 +105,14 @@ struct CfgXYV {
   static_assert(WB + TX - MX + WIN <= BW, "x window stays inside the staged row");
   static_assert(NTASK <= 2 * NT, "at most two x-pass tasks per thread");
 };
+
+// The kernels of one VJP are programmatic dependents of each other (and of the
+// stream's previous kernel): the next one's CTAs are scheduled as this one's
+// retire and wait here before they touch global memory.
+__device__ __forceinline__ void pdl_begin() {
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+}
 
 // x pass of one task (8 outputs of one staged row) in tap-pair form over the
 // zero-filled halo: with (we, wo) or (dwe, dwo).
@@ -154,6 +163,7 @@ __global__ void __launch_bounds__(256, 2)
   const int64_t u_begin = a.units * blockIdx.x / gridDim.x;
   const int64_t u_end = a.units * (blockIdx.x + 1) / gridDim.x;
   const uint64_t pol_in = policy_evict_first();
+  pdl_begin();
 
   const int row_a = tid / SEGS, x0_a = (tid % SEGS) * MX;
   const int row_b = (tid + NT) / SEGS, x0_b = ((tid + NT) % SEGS) * MX;
@@ -364,6 +374,26 @@ __global__ void __launch_bounds__(256, 2)
           }
         }
       }
+      // adjoint, accumulating: xbar's present values, all loads together before
+      // the stores (one by one, a load behind every store, they took the kernel
+      // from 25 to 36 us on 192^3, R = 6)
+      float2 old[MY];
+      if constexpr (MODE == kAdjoint) {
+#pragma unroll
+        for (int m = 0; m < MY; ++m) {
+          const int y = ty0 + grp * MY + m;
+          old[m] = make_float2(0.0f, 0.0f);
+          if (!a.accumulate || y > a.hi[1] || !c0ok) continue;
+          const float* const q = reinterpret_cast<const float*>(
+              a.out + (int64_t)(col - a.lo[0]) * 4 + (int64_t)(y - a.lo[1]) * a.out_pitch[1] + (int64_t)(sl - a.lo[2]) * a.out_pitch[2]);
+          if (c1ok && a.out_pair) {
+            old[m] = *reinterpret_cast<const float2*>(q);
+          } else {
+            old[m].x = q[0];
+            if (c1ok) old[m].y = q[1];
+          }
+        }
+      }
       // outputs: rows ty0 + grp*MY + m, columns col, col + 1 (inside the image only)
 #pragma unroll
       for (int m = 0; m < MY; ++m) {
@@ -375,13 +405,13 @@ __global__ void __launch_bounds__(256, 2)
           char* const p = a.out + (int64_t)(col - a.lo[0]) * a.out_pitch[0] + (int64_t)(y - a.lo[1]) * a.out_pitch[1] +
                           (int64_t)(sl - a.lo[2]) * a.out_pitch[2];
           float* const q0 = reinterpret_cast<float*>(p);
-          float* const q1 = reinterpret_cast<float*>(p + a.out_pitch[0]);
-          if (a.accumulate) {
-            v0 += *q0;
-            if (c1ok) v1 += *q1;
+          if (a.accumulate) v0 += old[m].x, v1 += old[m].y;
+          if (c1ok && a.out_pair) {
+            *reinterpret_cast<float2*>(q0) = make_float2(v0, v1);
+          } else {
+            q0[0] = v0;
+            if (c1ok) q0[1] = v1;
           }
-          *q0 = v0;
-          if (c1ok) *q1 = v1;
         } else {
           float d0, d1;
           unpack2(yd[m], d0, d1);
@@ -437,6 +467,7 @@ __global__ void __launch_bounds__(256, RZ <= 8 ? 2 : 1) k_z_adj(const __grid_con
   const uint32_t my_slot0 = smem_u32(zring + tid);
   const uint64_t pol = policy_evict_first();
   const int64_t nq = (int64_t)a.nqx * a.ny;
+  pdl_begin();
 
   for (int64_t u = u_begin; u < u_end;) {
     const int64_t blk = u / a.nz;
@@ -521,21 +552,26 @@ __global__ void __launch_bounds__(256, RZ <= 8 ? 2 : 1) k_z_adj(const __grid_con
 
 // Both z adjoints at once: U = Gz^T ybar and U' = dGz^T ybar from one pass over
 // ybar.  One thread marches one pair of columns (8-byte loads into its own
-// cp.async ring) with two rings of 2 RZ + 1 packed accumulators, one per
-// weight set; otherwise as k_z_adj.
-__device__ __forceinline__ void cp_async8(uint32_t s, const void* g) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(g) : "memory");
+// cp.async ring, zeros outside the image) with two rings of 2 RZ + 1 packed
+// accumulators, one per weight set.  The march carries no edge logic: the
+// clamped taps are folded onto the first and last slice afterwards, from
+// re-read slices.  CTAs' runs of slices as in k_z_pass (z_split).
+__device__ __forceinline__ void cp_async8_zfill(uint32_t s, const void* g, bool in) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(s), "l"(g), "r"(in ? 8 : 0) : "memory");
 }
 
+constexpr int kZ2Threads = 128;  // (blocks of 256 left room for 8 warps per SM from RZ = 7 on, these for 12)
+
 template <int RZ>
-__global__ void __launch_bounds__(256, RZ <= 6 ? 2 : 1) k_z_adj2(const __grid_constant__ ZAArgs a) {
-  constexpr int KZ = 2 * RZ + 1, S = KZ, NT = 256;
+__global__ void __launch_bounds__(kZ2Threads, RZ <= 6 ? 4 : RZ <= 9 ? 3 : 2) k_z_adj2(const __grid_constant__ ZAArgs a) {
+  constexpr int KZ = 2 * RZ + 1, S = KZ, NT = kZ2Threads;
   extern __shared__ __align__(16) float2 zring2[];  // [S][NT]
   const int tid = threadIdx.x;
-  const int64_t u_begin = a.units * blockIdx.x / gridDim.x;
-  const int64_t u_end = a.units * (blockIdx.x + 1) / gridDim.x;
+  const int64_t u_begin = a.nsplit > 0 ? (int64_t)a.split[blockIdx.x] : a.units * blockIdx.x / gridDim.x;
+  const int64_t u_end = a.nsplit > 0 ? (int64_t)a.split[blockIdx.x + 1] : a.units * (blockIdx.x + 1) / gridDim.x;
   const uint32_t my_slot0 = smem_u32(zring2 + tid);
   const int64_t np = (int64_t)a.npx * a.ny;
+  pdl_begin();
 
   for (int64_t u = u_begin; u < u_end;) {
     const int64_t blk = u / a.nz;
@@ -547,13 +583,14 @@ __global__ void __launch_bounds__(256, RZ <= 6 ? 2 : 1) k_z_adj2(const __grid_co
     if (q >= np) continue;
     const int cy = (int)(q / a.npx), px = (int)(q - (int64_t)cy * a.npx);
     const int cx = 2 * px;
-    const int jb = zs - RZ, je = ze - 1 + RZ;
     const char* const src = a.in + (int64_t)cx * a.in_pitch[0] + (int64_t)cy * a.in_pitch[1];
-    int jn = jb;
-    auto prefetch = [&](int stage) {  // slice jn, clamped to the image (a valid address)
-      cp_async8(my_slot0 + (uint32_t)(stage * NT * 8), src + (int64_t)clampi(jn, 0, a.nz - 1) * a.in_pitch[2]);
+    int jn = zs - RZ;  // next slice to fetch
+    const char* pn = src + (int64_t)clampi(jn, 0, a.nz - 1) * a.in_pitch[2];
+    auto prefetch = [&](int stage) {
+      cp_async8_zfill(my_slot0 + (uint32_t)(stage * NT * 8), pn, (unsigned)jn < (unsigned)a.nz);
       fusedk::cp_async_commit();
       ++jn;
+      pn += (unsigned)(jn - 1) < (unsigned)(a.nz - 1) ? a.in_pitch[2] : 0;  // slice jn - 1 -> jn inside the image
     };
 #pragma unroll
     for (int i = 0; i < S; ++i) prefetch(i);
@@ -562,61 +599,75 @@ __global__ void __launch_bounds__(256, RZ <= 6 ? 2 : 1) k_z_adj2(const __grid_co
     for (int m = 0; m < 2; ++m)
 #pragma unroll
       for (int k = 0; k < KZ; ++k) acc[m][k] = 0ull;
-    f2_t flo[2] = {0ull, 0ull}, fhi[2] = {0ull, 0ull};
     const bool two = cx + 1 < a.nx;
-    const int64_t ooff = (int64_t)cx * a.out_pitch[0] + (int64_t)cy * a.out_pitch[1] + (int64_t)zs * a.out_pitch[2];
-    char* dz = a.out + ooff;
-    char* dz2 = a.out2 + ooff;
-    for (int jbase = jb; jbase <= je; jbase += KZ) {
+    const int64_t ooff = (int64_t)cx * a.out_pitch[0] + (int64_t)cy * a.out_pitch[1];
+    char* const o1 = a.out + ooff;
+    char* const o2 = a.out2 + ooff;
+    char* dz = o1 + (int64_t)zs * a.out_pitch[2];
+    char* dz2 = o2 + (int64_t)zs * a.out_pitch[2];
+    auto step = [&](int p, bool store) {  // slice (period start) + p sits in stage p
+      fusedk::cp_async_wait<S - 1>();
+      const float2 f = zring2[p * NT + tid];
+      prefetch(p);
+      const f2_t v = pack2(f.x, f.y);
 #pragma unroll
-      for (int p = 0; p < KZ; ++p) {
-        const int j = jbase + p;
-        if (j > je) break;
-        fusedk::cp_async_wait<S - 1>();
-        const float2 f = zring2[p * NT + tid];
-        prefetch(p);
-        const bool inside = j >= 0 && j < a.nz;  // outside: zero (no contribution)
-        const f2_t v = inside ? pack2(f.x, f.y) : 0ull;
-#pragma unroll
-        for (int k = 0; k < KZ; ++k) {
-          const int slot = (p - k + KZ) % KZ;
-          const int kk = k <= RZ ? k : 2 * RZ - k;
-          acc[0][slot] = k == 0 ? mul2(v, a.wz2[kk]) : fma2(v, a.wz2[kk], acc[0][slot]);
-          acc[1][slot] = k == 0 ? mul2(v, a.wz2d[kk]) : fma2(v, a.wz2d[kk], acc[1][slot]);
-        }
-        // folds: the clamped taps of slices 0 .. R-1 onto slice 0, of the last R onto the last
-        if (inside && j < RZ) {
-          const float c = a.pz[RZ - j], cd = a.pzd[RZ - j];
-          flo[0] = fma2(v, pack2(c, c), flo[0]);
-          flo[1] = fma2(v, pack2(cd, cd), flo[1]);
-        }
-        if (inside && j > a.nz - 1 - RZ) {
-          const float c = a.pz[RZ - (a.nz - 1 - j)], cd = a.pzd[RZ - (a.nz - 1 - j)];
-          fhi[0] = fma2(v, pack2(c, c), fhi[0]);
-          fhi[1] = fma2(v, pack2(cd, cd), fhi[1]);
-        }
-        const int D = (p + 1) % KZ;
-        const int z = j - RZ;
-        if (z >= zs) {
-          f2_t d0 = acc[0][D], d1 = acc[1][D];
-          if (z == 0) d0 = add2(d0, flo[0]), d1 = add2(d1, flo[1]);
-          if (z == a.nz - 1) d0 = add2(d0, fhi[0]), d1 = add2(d1, fhi[1]);
-          float o0, o1, e0, e1;
-          unpack2(d0, o0, o1);
-          unpack2(d1, e0, e1);
-          if (two) {
-            *reinterpret_cast<float2*>(dz) = make_float2(o0, o1);
-            *reinterpret_cast<float2*>(dz2) = make_float2(e0, e1);
-          } else {
-            *reinterpret_cast<float*>(dz) = o0;
-            *reinterpret_cast<float*>(dz2) = e0;
-          }
-          dz += a.out_pitch[2];
-          dz2 += a.out_pitch[2];
-        }
+      for (int k = 0; k < KZ; ++k) {
+        const int slot = (p - k + KZ) % KZ;
+        const int kk = k <= RZ ? k : 2 * RZ - k;
+        acc[0][slot] = k == 0 ? mul2(v, a.wz2[kk]) : fma2(v, a.wz2[kk], acc[0][slot]);
+        acc[1][slot] = k == 0 ? mul2(v, a.wz2d[kk]) : fma2(v, a.wz2d[kk], acc[1][slot]);
       }
+      if (!store) return;
+      const int D = (p + 1) % KZ;
+      float c0, c1, e0, e1;
+      unpack2(acc[0][D], c0, c1);
+      unpack2(acc[1][D], e0, e1);
+      if (two) {
+        *reinterpret_cast<float2*>(dz) = make_float2(c0, c1);
+        *reinterpret_cast<float2*>(dz2) = make_float2(e0, e1);
+      } else {
+        *reinterpret_cast<float*>(dz) = c0;
+        *reinterpret_cast<float*>(dz2) = e0;
+      }
+      dz += a.out_pitch[2];
+      dz2 += a.out_pitch[2];
+    };
+    // first period: slices zs - RZ .. zs + RZ; only the last one completes an output (zs)
+#pragma unroll
+    for (int p = 0; p < KZ; ++p) step(p, p == KZ - 1);
+    const int rest = ze - zs - 1;
+    const int nfull = rest / KZ, tail = rest - nfull * KZ;
+    for (int it = 0; it < nfull; ++it) {
+#pragma unroll
+      for (int p = 0; p < KZ; ++p) step(p, true);
+    }
+#pragma unroll
+    for (int p = 0; p < KZ; ++p) {
+      if (p >= tail) break;
+      step(p, true);
     }
     fusedk::cp_async_wait<0>();
+    // folds: the clamped taps of slices 0 .. R-1 onto slice 0, of the last R onto the last
+    auto fold = [&](int z, int j0, int j1, bool low) {
+      f2_t f1 = 0ull, f2 = 0ull;
+      for (int j = j0; j < j1; ++j) {
+        const char* const g = src + (int64_t)j * a.in_pitch[2];
+        const f2_t v = two ? *reinterpret_cast<const f2_t*>(g) : pack2(*reinterpret_cast<const float*>(g), 0.0f);
+        const int i = low ? RZ - j : RZ - (a.nz - 1 - j);
+        const float c = a.pz[i], cd = a.pzd[i];
+        f1 = fma2(v, pack2(c, c), f1);
+        f2 = fma2(v, pack2(cd, cd), f2);
+      }
+      float* const p1 = reinterpret_cast<float*>(o1 + (int64_t)z * a.out_pitch[2]);
+      float* const p2 = reinterpret_cast<float*>(o2 + (int64_t)z * a.out_pitch[2]);
+      float l1, h1, l2, h2;
+      unpack2(f1, l1, h1);
+      unpack2(f2, l2, h2);
+      p1[0] += l1, p2[0] += l2;
+      if (two) p1[1] += h1, p2[1] += h2;
+    };
+    if (zs == 0) fold(0, 0, min(RZ, a.nz), true);
+    if (ze == a.nz) fold(a.nz - 1, max(0, a.nz - RZ), a.nz, false);
   }
 }
 
