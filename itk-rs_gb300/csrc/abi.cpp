@@ -430,6 +430,10 @@ static itkg_status generate_device(const itkg_image& in, const itkg_region& larg
     std::vector<float> c[kMaxDim];
     bool ok = true;
     for (int d = 0; d < D && ok; ++d) {
+      if (d > 0 && plan.w64[d] == plan.w64[d - 1]) {  // one kernel for several axes: its constants are found once
+        c[d] = c[d - 1];
+        continue;
+      }
       c[d].resize(plan.w64[d].size());
       ok = u8_pixel_tap_consts(plan.w64[d].data(), (int)plan.w64[d].size(), c[d].data());
     }

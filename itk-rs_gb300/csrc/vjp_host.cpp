@@ -189,6 +189,21 @@ DotArgs dot_args(const itkg_image& p, const itkg_image& q) {
   return d;
 }
 
+// Reads n doubles from the device after the work queued on s, through a pinned
+// buffer of the calling thread (a copy to pageable memory is staged by the
+// driver and cost a single result 8 us more).  Synchronises s.
+constexpr int kPinnedDoubles = 64;
+itkg_status read_back(const double* dev, int n, double* out, cudaStream_t s) {
+  thread_local double* pinned = nullptr;
+  if (n <= kPinnedDoubles && !pinned)
+    ITKG_CUDA(cudaMallocHost(reinterpret_cast<void**>(&pinned), sizeof(double) * kPinnedDoubles));
+  double* const to = n <= kPinnedDoubles ? pinned : out;
+  ITKG_CUDA(cudaMemcpyAsync(to, dev, sizeof(double) * (size_t)n, cudaMemcpyDeviceToHost, s));
+  ITKG_CUDA(cudaStreamSynchronize(s));
+  if (to != out) std::memcpy(out, to, sizeof(double) * (size_t)n);
+  return ITKG_SUCCESS;
+}
+
 // Fused geometry of a whole-image VJP launch: src over its own region, the
 // request and the clamp bounds both the whole image.
 FusedGeom whole_geom(const itkg_image& src, const itkg_image* dst, const AxisCoeffs* c) {
@@ -291,8 +306,7 @@ extern "C" itkg_status itkg_gaussian_scale_stack_loss_vjp(
   }
   if (loss || (sigma_bar && !on_dev)) {
     std::vector<double> h(1 + nlevels);
-    ITKG_CUDA(cudaMemcpyAsync(h.data(), dloss, sizeof(double) * (1 + nlevels), cudaMemcpyDeviceToHost, s));
-    ITKG_CUDA(cudaStreamSynchronize(s));
+    ITKG_TRY(read_back(dloss, 1 + nlevels, h.data(), s));
     if (loss) *loss = h[0];
     if (sigma_bar && !on_dev)
       for (int l = 0; l < nlevels; ++l) sigma_bar[l] = h[1 + l];
@@ -354,8 +368,7 @@ extern "C" itkg_status itkg_gaussian_vjp(const itkg_image* x, const itkg_image* 
       ITKG_TRY(launch_vjp_two_pass(v, s, false));
       if (sigma_bar && !on_dev) {
         double h = 0.0;
-        ITKG_CUDA(cudaMemcpyAsync(&h, dres, sizeof h, cudaMemcpyDeviceToHost, s));
-        ITKG_CUDA(cudaStreamSynchronize(s));
+        ITKG_TRY(read_back(dres, 1, &h, s));
         *sigma_bar = (flags & ITKG_VJP_ACCUMULATE_SIGMA) ? *sigma_bar + h : h;
       }
       set_last_kernel("vjp_two_pass_f32");
@@ -411,8 +424,7 @@ extern "C" itkg_status itkg_gaussian_vjp(const itkg_image* x, const itkg_image* 
     }
     if (!on_dev) {
       double h = 0.0;
-      ITKG_CUDA(cudaMemcpyAsync(&h, dres, sizeof h, cudaMemcpyDeviceToHost, s));
-      ITKG_CUDA(cudaStreamSynchronize(s));
+      ITKG_TRY(read_back(dres, 1, &h, s));
       *sigma_bar = acc ? *sigma_bar + h : h;
     }
   }

@@ -100,6 +100,18 @@ class Region:
             r.size[d] = int(self.size[d]) if d < self.dim else 1
         return r
 
+    def _c(self) -> itkg_region:
+        """to_c() for read-only use: built once for a region of tuples, which cannot change."""
+        r = self.__dict__.get("_c_struct")
+        if r is None:
+            r = self.to_c()
+            if type(self.index) is tuple and type(self.size) is tuple:
+                self.__dict__["_c_struct"] = r
+        return r
+
+    def __reduce__(self):
+        return Region, (self.index, self.size)
+
     @staticmethod
     def from_c(r: itkg_region, dim: int) -> "Region":
         return Region(tuple(r.index[d] for d in range(dim)), tuple(r.size[d] for d in range(dim)))
@@ -350,11 +362,10 @@ class GaussianFilter:
                         out_dtype: int | None = None, out=None):
         """Returns a host Image for a host source, a DeviceImage for a device source."""
         leaf = self._leaf()
-        prm = self.params()
         if out_dtype is None:
-            out_dtype = U8 if prm.arithmetic == ARITH_PIXEL_U8 else F32
-        largest = leaf.largest_region().to_c()
-        req = requested.to_c()
+            out_dtype = U8 if self.params().arithmetic == ARITH_PIXEL_U8 else F32
+        largest = leaf.largest_region()._c()
+        req = requested._c()
         src = leaf.to_c()
         if isinstance(leaf, Image):
             shape = tuple(reversed(requested.size)) + ((leaf.components,) if leaf.components > 1 else ())
@@ -716,8 +727,8 @@ class RecursiveGaussianFilter:
         if out_dtype is None:
             out_dtype = U8 if src.dtype == U8 else F32
         prm = self.params()
-        largest = src.largest_region().to_c()
-        req = requested.to_c()
+        largest = src.largest_region()._c()
+        req = requested._c()
         sc = src.to_c()
         if isinstance(src, Image):
             host = np.empty(tuple(reversed(requested.size)), dtype=_storage_np(out_dtype))
@@ -765,8 +776,8 @@ class RecursiveGaussianDerivativeFilter(RecursiveGaussianFilter):
         p = itkg_recursive_derivative_params()
         p.sigma, p.kind, p.axis, p.order, p.rounding = self.sigma, self.kind, self.deriv_axis, self.order, self.rounding
         p.sigma2 = self.sigma2
-        largest = src.largest_region().to_c()
-        req = requested.to_c()
+        largest = src.largest_region()._c()
+        req = requested._c()
         sc = src.to_c()
         if isinstance(src, Image):
             shape = tuple(reversed(requested.size)) + ((comps,) if comps > 1 else ())
