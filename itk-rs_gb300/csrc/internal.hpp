@@ -335,13 +335,12 @@ itkg_status launch_dot(const DotArgs& d, double* partials, int nblocks, double* 
 // *out (+)= sum of n f64 partials, in a fixed order.
 itkg_status launch_sum_partials(const double* partials, int n, double* out, bool accumulate,
                                 void* stream);
-// Squared error against t (DotArgs::q / q_pitch / size): ybar = 2 (y - t) into
-// a dense buffer; *loss_out (+)= sum (y - t)^2, *sigma_out = sum ybar * dy
-// (dy and sigma_out may be NULL: no sigma term).
-// partials: 2 * nblocks doubles of scratch.  y, dy, ybar dense f32.
-itkg_status launch_sqerr(const float* y, const float* dy, const DotArgs& t, float* ybar,
-                         double* partials, int nblocks, double* loss_out, double* sigma_out,
-                         bool accumulate_loss, void* stream);
+// Squared error against t (DotArgs::q / q_pitch / size): ybar = 2 (y - t), and
+// per block the sums of (y - t)^2 and of ybar * dy (0 with dy NULL) into
+// loss_part / sig_part.  *nblocks: room in each; lowered to the blocks used.
+// y, dy, ybar: f32 rows of `row_floats` floats, dense otherwise.
+itkg_status launch_sqerr(const float* y, const float* dy, const DotArgs& t, float* ybar, int64_t row_floats,
+                         double* loss_part, double* sig_part, int* nblocks, void* stream);
 
 // Clock cycles a kernel's bounded wait on a tile load may take before it
 // gives up (abi.cpp; 2^31 unless a test lowered it).

@@ -321,7 +321,8 @@ __global__ void __launch_bounds__(kThreads) k_dot_partials(const DotArgs d, doub
 // relative error near 1e-7).
 __global__ void __launch_bounds__(kThreads) k_sqerr(const float* __restrict__ y,
                                                      const float* __restrict__ dy, const DotArgs t,
-                                                     float* __restrict__ ybar, double* partials) {
+                                                     float* __restrict__ ybar, int64_t pitch, double* loss_part,
+                                                     double* sig_part) {
   const int64_t nx = t.size[0], ny = t.size[1];
   const int64_t rows = ny * t.size[2];
   const int64_t r0 = rows * blockIdx.x / gridDim.x, r1 = rows * (blockIdx.x + 1) / gridDim.x;
@@ -331,7 +332,7 @@ __global__ void __launch_bounds__(kThreads) k_sqerr(const float* __restrict__ y,
   for (int64_t row = r0; row < r1; ++row) {
     const int64_t yy = row % ny, z = row / ny;
     const char* const trow = reinterpret_cast<const char*>(t.q) + yy * t.q_pitch[1] + z * t.q_pitch[2];
-    const int64_t base = row * nx;
+    const int64_t base = row * pitch;
     for (int64_t x = threadIdx.x; x < nx; x += kThreads) {
       const float tv = *reinterpret_cast<const float*>(trow + x * t.q_pitch[0]);
       const float d = y[base + x] - tv;
@@ -361,40 +362,69 @@ __global__ void __launch_bounds__(kThreads) k_sqerr(const float* __restrict__ y,
     __syncthreads();
   }
   if (threadIdx.x == 0) {
-    partials[blockIdx.x] = red[0][0];
-    partials[gridDim.x + blockIdx.x] = red[1][0];
+    loss_part[blockIdx.x] = red[0][0];
+    sig_part[blockIdx.x] = red[1][0];
   }
 }
 
-// The same over dense images whose rows are whole quads (the target too): a
-// grid-stride loop over the volume's quads, four quads per thread in flight,
-// the f32 runs folded into f64 every 8 quads.  A fixed grid makes the partials
-// deterministic.
-__global__ void __launch_bounds__(kThreads) k_sqerr_q(const float4* __restrict__ y, const float4* __restrict__ dy,
-                                                        const float4* __restrict__ t, float4* __restrict__ ybar,
-                                                        int64_t nq, double* partials) {
+// The same over rows on 16-byte boundaries (the target's too): a grid-stride
+// loop over the volume's quads, four quads per thread in flight, the f32 runs
+// folded into f64 every 4 quads; the last quad of a row may be partial.  A fixed
+// grid makes the partials deterministic.
+struct SqerrRows {
+  const float* y;   // y, dy and ybar share one layout: rows of `pitch` quads
+  const float* dy;  // may be NULL
+  float* ybar;
+  const char* t;    // the target and its byte pitches
+  int64_t t1, t2;
+  uint32_t nx, ny, nqx, pitch;  // row length, rows per slice, quads per row, quads between rows
+  uint32_t total;   // quads
+};
+
+__device__ __forceinline__ float4 quad_of(const float* p, int n) {  // the first n floats, zeros after them
+  if (n == 4) return *reinterpret_cast<const float4*>(p);
+  return make_float4(p[0], n > 1 ? p[1] : 0.0f, n > 2 ? p[2] : 0.0f, 0.0f);
+}
+
+__global__ void __launch_bounds__(kThreads) k_sqerr_q(const __grid_constant__ SqerrRows a, double* loss_part,
+                                                        double* sig_part) {
   constexpr int U = 4;
+  // a programmatic dependent of the forward's last kernel; the VJP's first one may follow likewise
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
   double sl = 0.0, ss = 0.0;
-  const int64_t stride = (int64_t)gridDim.x * kThreads;
-  for (int64_t i0 = (int64_t)blockIdx.x * kThreads + threadIdx.x; i0 < nq; i0 += U * stride) {
+  const uint32_t stride = gridDim.x * kThreads;
+  for (uint32_t i0 = blockIdx.x * kThreads + threadIdx.x; i0 < a.total; i0 += U * stride) {
     float4 yv[U], tv[U], dv[U];
+    int64_t at[U];
+    int nc[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int64_t i = i0 + u * stride;
-      if (i < nq) {
-        yv[u] = __ldcs(y + i);
-        tv[u] = __ldg(t + i);
-        dv[u] = dy ? __ldcs(dy + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      const uint32_t i = i0 + u * stride;
+      nc[u] = 0;
+      if (i < a.total) {
+        const uint32_t row = i / a.nqx, qx = i - row * a.nqx, z = row / a.ny, y = row - z * a.ny;
+        at[u] = ((int64_t)row * a.pitch + qx) * 4;
+        nc[u] = (int)min(4u, a.nx - 4 * qx);
+        yv[u] = quad_of(a.y + at[u], nc[u]);
+        tv[u] = quad_of(reinterpret_cast<const float*>(a.t + y * a.t1 + z * a.t2) + 4 * qx, nc[u]);
+        dv[u] = a.dy ? quad_of(a.dy + at[u], nc[u]) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
       }
     }
     float fl = 0.0f, fs = 0.0f;
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int64_t i = i0 + u * stride;
-      if (i >= nq) break;
+      if (nc[u] == 0) break;
+      // (a partial quad's missing values are zeros throughout)
       const float4 d = make_float4(yv[u].x - tv[u].x, yv[u].y - tv[u].y, yv[u].z - tv[u].z, yv[u].w - tv[u].w);
       const float4 g = make_float4(2.0f * d.x, 2.0f * d.y, 2.0f * d.z, 2.0f * d.w);
-      __stcs(ybar + i, g);
+      if (nc[u] == 4) {
+        __stcs(reinterpret_cast<float4*>(a.ybar + at[u]), g);
+      } else {
+        a.ybar[at[u]] = g.x;
+        if (nc[u] > 1) a.ybar[at[u] + 1] = g.y;
+        if (nc[u] > 2) a.ybar[at[u] + 2] = g.z;
+      }
       fl = fmaf(d.x, d.x, fl);
       fl = fmaf(d.y, d.y, fl);
       fl = fmaf(d.z, d.z, fl);
@@ -419,8 +449,8 @@ __global__ void __launch_bounds__(kThreads) k_sqerr_q(const float4* __restrict__
     __syncthreads();
   }
   if (threadIdx.x == 0) {
-    partials[blockIdx.x] = red[0][0];
-    partials[gridDim.x + blockIdx.x] = red[1][0];
+    loss_part[blockIdx.x] = red[0][0];
+    sig_part[blockIdx.x] = red[1][0];
   }
 }
 
@@ -505,30 +535,39 @@ int dot_partial_blocks(int64_t n) {
   return (int)(b < 1 ? 1 : (b > 2048 ? 2048 : b));
 }
 
-itkg_status launch_sqerr(const float* y, const float* dy, const DotArgs& t, float* ybar,
-                         double* partials, int nblocks, double* loss_out, double* sigma_out,
-                         bool accumulate_loss, void* stream) {
+itkg_status launch_sqerr(const float* y, const float* dy, const DotArgs& t, float* ybar, int64_t row_floats,
+                         double* loss_part, double* sig_part, int* nblocks, void* stream) {
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const int64_t nx = t.size[0], ny = t.size[1];
-  const bool quads = nx % 4 == 0 && t.q_pitch[0] == 4 && t.q_pitch[1] == 4 * nx && t.q_pitch[2] == 4 * nx * ny &&
-                     (((uintptr_t)y | (uintptr_t)dy | (uintptr_t)t.q | (uintptr_t)ybar) & 15) == 0;
-  // the quad kernel: about 16 quads per thread (fewer, longer-running blocks)
-  const int64_t nq = nx / 4 * ny * t.size[2];
-  const int nb = quads ? (int)std::max<int64_t>(1, std::min<int64_t>(nblocks, (nq + kThreads * 16 - 1) / (kThreads * 16)))
-                       : nblocks;
-  if (quads)
-    k_sqerr_q<<<nb, kThreads, 0, s>>>(reinterpret_cast<const float4*>(y), reinterpret_cast<const float4*>(dy),
-                                      reinterpret_cast<const float4*>(t.q), reinterpret_cast<float4*>(ybar), nq,
-                                      partials);
-  else
-    k_sqerr<<<nb, kThreads, 0, s>>>(y, dy, t, ybar, partials);
-  itkg_status st = launched("sqerr_partials_f64");
-  if (st != ITKG_SUCCESS) return st;
-  k_sum_partials<<<1, kThreads, 0, s>>>(partials, nb, loss_out, accumulate_loss ? 1 : 0);
-  if ((st = launched("sum_partials_f64")) != ITKG_SUCCESS) return st;
-  if (!sigma_out) return ITKG_SUCCESS;
-  k_sum_partials<<<1, kThreads, 0, s>>>(partials + nb, nb, sigma_out, 0);
-  return launched("sum_partials_f64");
+  const int64_t nx = t.size[0], ny = t.size[1], nz = t.size[2];
+  const int64_t nqx = (nx + 3) / 4, nq = nqx * ny * nz;
+  const bool quads = row_floats % 4 == 0 && t.q_pitch[0] == 4 && t.q_pitch[1] % 16 == 0 && t.q_pitch[2] % 16 == 0 &&
+                     (((uintptr_t)y | (uintptr_t)dy | (uintptr_t)t.q | (uintptr_t)ybar) & 15) == 0 &&
+                     nq < INT32_MAX && ny <= INT32_MAX && row_floats / 4 <= INT32_MAX;
+  if (quads) {
+    // about 16 quads per thread (fewer, longer-running blocks)
+    *nblocks = (int)std::max<int64_t>(1, std::min<int64_t>(*nblocks, (nq + kThreads * 16 - 1) / (kThreads * 16)));
+    SqerrRows a;
+    a.y = y, a.dy = dy, a.ybar = ybar;
+    a.t = reinterpret_cast<const char*>(t.q);
+    a.t1 = t.q_pitch[1], a.t2 = t.q_pitch[2];
+    a.nx = (uint32_t)nx, a.ny = (uint32_t)ny, a.nqx = (uint32_t)nqx, a.pitch = (uint32_t)(row_floats / 4);
+    a.total = (uint32_t)nq;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg;
+    std::memset(&cfg, 0, sizeof cfg);
+    cfg.gridDim = dim3((unsigned)*nblocks);
+    cfg.blockDim = dim3(kThreads);
+    cfg.stream = s;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, k_sqerr_q, a, loss_part, sig_part);
+    if (e != cudaSuccess) return set_error(ITKG_ERROR_CUDA, "sqerr_partials_f64 launch: %s", cudaGetErrorString(e));
+  } else {
+    k_sqerr<<<*nblocks, kThreads, 0, s>>>(y, dy, t, ybar, row_floats, loss_part, sig_part);
+  }
+  return launched("sqerr_partials_f64");
 }
 
 itkg_status launch_sum_partials(const double* partials, int n, double* out, bool accumulate,

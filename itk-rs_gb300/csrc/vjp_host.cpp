@@ -77,7 +77,7 @@ void view3(const itkg_image& im, int64_t* pitch, int64_t* size) {
   }
 }
 
-// Scratch images: dense f32 of the same size.
+// Scratch images: f32 of the same size, rows on 16-byte boundaries.
 struct Scratch {
   std::vector<void*> ptrs;
   cudaStream_t s;
@@ -92,7 +92,7 @@ struct Scratch {
     out->components = 1;
     out->location = ITKG_DEVICE;
     out->region = like.region;
-    dense_layout(out, 1);  // fully dense: the loss kernel indexes it linearly
+    dense_layout(out, 16);
     void* p = nullptr;
     ITKG_TRY(scratch_alloc(&p, image_bytes(*out), s));
     ptrs.push_back(p);
@@ -204,6 +204,10 @@ itkg_status read_back(const double* dev, int n, double* out, cudaStream_t s) {
   return ITKG_SUCCESS;
 }
 
+// Fewest voxels with rows of no multiple of 4 floats whose levels take the
+// two-pass kernels.
+constexpr int64_t kRaggedTwoPass = 1 << 14;
+
 // Fused geometry of a whole-image VJP launch: src over its own region, the
 // request and the clamp bounds both the whole image.
 FusedGeom whole_geom(const itkg_image& src, const itkg_image* dst, const AxisCoeffs* c) {
@@ -262,20 +266,26 @@ extern "C" itkg_status itkg_gaussian_scale_stack_loss_vjp(
   ITKG_TRY(sc.image(*x, &dy));
   ITKG_TRY(sc.image(*x, &yb));
   const int nb = dot_partial_blocks(n);
+  const int64_t row_floats = y.pitch[1] / 4;
+  // the loss partials of every level side by side (summed once, at the end),
+  // the sigma partials of one level, then the results
   void* part = nullptr;
-  ITKG_TRY(sc.raw(sizeof(double) * (2 * nb + 1 + nlevels), &part));
-  double* partials = static_cast<double*>(part);
-  double* dloss = partials + 2 * nb;
+  ITKG_TRY(sc.raw(sizeof(double) * ((size_t)nb * ((size_t)nlevels + 1) + 1 + (size_t)nlevels), &part));
+  double* loss_part = static_cast<double*>(part);
+  double* const sig_part = loss_part + (size_t)nb * (size_t)nlevels;
+  double* dloss = sig_part + nb;
   double* dsig = dloss + 1;
+  int64_t nloss = 0;
   const bool on_dev = flags & ITKG_VJP_SIGMA_BAR_ON_DEVICE;
   int fast_levels = 0;
   for (int l = 0; l < nlevels; ++l) {
     const AxisCoeffs* c = &coeffs[(size_t)l * kMaxDim];
     double* const sig_l = on_dev && sigma_bar ? sigma_bar + l : dsig + l;
     DotArgs t = dot_args(y, *target);  // q = target
-    // Two-pass forward and VJP kernels where they apply (3-D, the dense scratch
-    // rows 16-byte aligned): y_l, then ybar_l = 2 (y_l - t), then xbar and
-    // dL/dsigma_l from the VJP kernels.
+    // Two-pass forward and VJP kernels where they apply (3-D): y_l, then
+    // ybar_l = 2 (y_l - t), then xbar and dL/dsigma_l from the VJP kernels.
+    // Images of a few thousand voxels with ragged rows stay with the per-axis
+    // passes.
     VjpTwoPass v;
     v.x = x;
     v.ybar = &yb;
@@ -284,7 +294,9 @@ extern "C" itkg_status itkg_gaussian_scale_stack_loss_vjp(
     v.acc_x = l > 0;
     v.acc_sigma = false;
     for (int d = 0; d < x->dim; ++d) v.w[d] = c[d].w.data(), v.dw[d] = c[d].dw.data(), v.radius[d] = (int)c[d].r;
-    if (x->dim == 3 && x->region.size[0] % 4 == 0 && launch_vjp_two_pass(v, s, true) == ITKG_SUCCESS) {
+    int blocks = nb;
+    if (x->dim == 3 && (x->region.size[0] % 4 == 0 || n >= kRaggedTwoPass) &&
+        launch_vjp_two_pass(v, s, true) == ITKG_SUCCESS) {
       itkg_gaussian_params p;
       std::memset(&p, 0, sizeof p);
       p.sigma = sigmas[l];
@@ -293,17 +305,21 @@ extern "C" itkg_status itkg_gaussian_scale_stack_loss_vjp(
       p.algorithm = ITKG_ALGO_AUTO;
       const itkg_region reg = x->region;
       ITKG_TRY(itkg_gaussian_generate_region(x, &reg, &reg, &p, &y, s));
-      ITKG_TRY(launch_sqerr(static_cast<const float*>(y.data), nullptr, t, static_cast<float*>(yb.data),
-                            partials, nb, dloss, nullptr, l > 0, s));
+      ITKG_TRY(launch_sqerr(static_cast<const float*>(y.data), nullptr, t, static_cast<float*>(yb.data), row_floats,
+                            loss_part + nloss, sig_part, &blocks, s));
+      nloss += blocks;
       ITKG_TRY(launch_vjp_two_pass(v, s, false));
       ++fast_levels;
       continue;
     }
     ITKG_TRY(dual_chain(*x, c, &y, &dy, sc));  // y_l and dy_l/dsigma_l, recomputed
     ITKG_TRY(launch_sqerr(static_cast<const float*>(y.data), static_cast<const float*>(dy.data), t,
-                          static_cast<float*>(yb.data), partials, nb, dloss, sig_l, l > 0, s));
+                          static_cast<float*>(yb.data), row_floats, loss_part + nloss, sig_part, &blocks, s));
+    nloss += blocks;
+    ITKG_TRY(launch_sum_partials(sig_part, blocks, sig_l, false, s));
     if (xbar) ITKG_TRY(adjoint_chain(yb, c, xbar, l > 0, sc));
   }
+  ITKG_TRY(launch_sum_partials(loss_part, (int)nloss, dloss, false, s));
   if (loss || (sigma_bar && !on_dev)) {
     std::vector<double> h(1 + nlevels);
     ITKG_TRY(read_back(dloss, 1 + nlevels, h.data(), s));
