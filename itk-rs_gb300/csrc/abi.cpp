@@ -464,6 +464,16 @@ static itkg_status generate_device(const itkg_image& in, const itkg_region& larg
       return launch_fused2d(g, w, s, false);
     itkg_status st = launch_fused(g, w, s, /*dry_run=*/true);
     if (st == ITKG_SUCCESS) return launch_fused(g, w, s, false);
+    // 2-D u8 images behind a cast to f32: the tile kernel while the per-axis
+    // passes would run tap by tap (radius below 8: 1601 x 1067, radius 5, 12.7
+    // against 58 us, 3 components 34 against 152), and for one component up to
+    // a megapixel (512^2, radius 9: 8.7 against 11.3 us, mostly launches); the
+    // line passes beyond (1601 x 1067, radius 9, 3 components: 35 against 50 us,
+    // the tiles' halo rows).
+    const bool tiles = plan.radii[0] < 8 ||
+                       (in.components == 1 && region_len(requested, D) <= (1ull << 20));
+    if (D == 2 && tiles && prm.algorithm == ITKG_ALGO_AUTO && launch_tile2d_u8(g, w, s, /*dry_run=*/true) == ITKG_SUCCESS)
+      return launch_tile2d_u8(g, w, s, false);
     if (prm.algorithm == ITKG_ALGO_FUSED)
       return set_error(ITKG_ERROR_UNSUPPORTED, "no fused kernel covers this geometry");
   }

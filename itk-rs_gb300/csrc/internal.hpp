@@ -126,6 +126,9 @@ itkg_status launch_fused2d(const FusedGeom& g, const float* const w[kMaxDim], vo
 // tile2d.cu: the same geometries on 64 x 32 tiles staged at once (small and
 // medium images); launch_fused2d chooses between the two.
 itkg_status launch_tile2d(const FusedGeom& g, const float* const w[kMaxDim], void* stream, bool dry_run);
+// tile2d.cu: the same from u8 pixels of 1 or 3 components in f32 arithmetic (any
+// output type); only the automatic choice takes it.
+itkg_status launch_tile2d_u8(const FusedGeom& g, const float* const w[kMaxDim], void* stream, bool dry_run);
 // tile2d.cu: many 2-D requests as one tile-kernel launch per kernel class
 // (radius, components, rounding); the batch's 2-D items.
 struct Tile2DMultiPlan;

@@ -74,7 +74,7 @@ __device__ __forceinline__ void cp4(float* dst, const void* src) {
 }
 
 // One tile t of the launch described by `a` (weights wx / wy in registers).
-template <int R, int C, bool REF>
+template <int R, int C, bool REF, typename Tin = float>
 __device__ __forceinline__ void tile2d_body(const Tile2DArgs& a, const float (&wx)[2 * R + 1],
                                             const float (&wy)[2 * R + 1], int64_t t, float* sm) {
   using G = T2Cfg<R, C>;
@@ -89,16 +89,41 @@ __device__ __forceinline__ void tile2d_body(const Tile2DArgs& a, const float (&w
   const char* const srcz = a.src + zq * a.src_slice;
 
   // 1. stage the clamped input tile; components fastest, so a warp reads
-  //    consecutive floats of an interleaved row
-  for (int e = threadIdx.x; e < IH * IW * C; e += kT2Threads) {
-    const int c = C == 1 ? 0 : e % C;
-    const int pe = C == 1 ? e : e / C;
-    const int col = pe % IW, row = pe / IW;
-    const int gx = min(max(tx0 - R + col, a.lo[0]), a.hi[0]);
-    const int gy = min(max(ty0 - R + row, a.lo[1]), a.hi[1]);
-    const char* p = srcz + (int64_t)(gx - a.src_origin[0]) * a.src_pitch[0] +
-                    (int64_t)(gy - a.src_origin[1]) * a.src_pitch[1] + c * 4;
-    cp4(sin + (c * IH + row) * IWP + col, p);
+  //    consecutive values of an interleaved row
+  constexpr int E = (int)sizeof(Tin);
+  const int px0 = tx0 - R;  // first staged pixel
+  if (E == 1 && px0 - 3 >= a.lo[0] && px0 + IW + 2 <= a.hi[0]) {
+    // u8 rows away from the x edges: aligned 4-byte words (up to 3 bytes more
+    // on either side, of the same row), converted as they are stored
+    constexpr int NB = IW * C;          // bytes of a staged row
+    constexpr int NW = (NB + 3) / 4 + 1;
+    for (int e = threadIdx.x; e < IH * NW; e += kT2Threads) {
+      const int row = e / NW, j = e - row * NW;
+      const int gy = min(max(ty0 - R + row, a.lo[1]), a.hi[1]);
+      const char* const p = srcz + (int64_t)(px0 - a.src_origin[0]) * C + (int64_t)(gy - a.src_origin[1]) * a.src_pitch[1];
+      const int shift = (int)(reinterpret_cast<uintptr_t>(p) & 3);
+      const int b0 = 4 * j - shift;  // the word's first byte in the row
+      if (b0 >= NB) continue;
+      const uint32_t v = __ldg(reinterpret_cast<const uint32_t*>(p + b0));
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int b = b0 + i;
+        if (b >= 0 && b < NB) sin[(b % C * IH + row) * IWP + b / C] = (float)((v >> (8 * i)) & 255u);
+      }
+    }
+  } else {
+    for (int e = threadIdx.x; e < IH * IW * C; e += kT2Threads) {
+      const int c = C == 1 ? 0 : e % C;
+      const int pe = C == 1 ? e : e / C;
+      const int col = pe % IW, row = pe / IW;
+      const int gx = min(max(px0 + col, a.lo[0]), a.hi[0]);
+      const int gy = min(max(ty0 - R + row, a.lo[1]), a.hi[1]);
+      const char* p = srcz + (int64_t)(gx - a.src_origin[0]) * a.src_pitch[0] +
+                      (int64_t)(gy - a.src_origin[1]) * a.src_pitch[1] + c * E;
+      float* const d = sin + (c * IH + row) * IWP + col;
+      if constexpr (E == 4) cp4(d, p);
+      else *d = to_f32(*reinterpret_cast<const Tin*>(p));
+    }
   }
   asm volatile("cp.async.wait_all;\n" ::: "memory");
   __syncthreads();
@@ -168,6 +193,16 @@ __global__ void __launch_bounds__(kT2Threads) k_tile2d(const Tile2DArgs a) {
   tile2d_body<R, C, REF>(a, wx, wy, blockIdx.x, sm);
 }
 
+// The same from u8 pixels (the cast of examples/blur_png.rs:35-37 on load).
+template <int R, int C, bool REF>
+__global__ void __launch_bounds__(kT2Threads) k_tile2d_u8(const Tile2DArgs a) {
+  extern __shared__ __align__(16) float sm[];
+  float wx[2 * R + 1], wy[2 * R + 1];
+#pragma unroll
+  for (int k = 0; k < 2 * R + 1; ++k) wx[k] = a.wx[k], wy[k] = a.wy[k];
+  tile2d_body<R, C, REF, uint8_t>(a, wx, wy, blockIdx.x, sm);
+}
+
 // Many requests of one class (radius, components, rounding) in one launch:
 // request q owns the CTAs [starts[q], starts[q + 1]); each CTA copies its
 // request's arguments to shared memory and its weights to registers.
@@ -222,6 +257,18 @@ const EntryT2 kTableT2[] = {
     make_t2<7, 2>(),  make_t2<8, 2>(),  make_t2<9, 2>(),  make_t2<10, 2>(), make_t2<11, 2>(), make_t2<12, 2>(),
 };
 
+template <int R, int C>
+EntryT2 make_t2u8() {
+  return EntryT2{R, C, {k_tile2d_u8<R, C, false>, k_tile2d_u8<R, C, true>}, {nullptr, nullptr}, T2Cfg<R, C>::SMEM};
+}
+const EntryT2 kTableT2U8[] = {
+    make_t2u8<1, 1>(),  make_t2u8<2, 1>(),  make_t2u8<3, 1>(),  make_t2u8<4, 1>(),  make_t2u8<5, 1>(),
+    make_t2u8<6, 1>(),  make_t2u8<7, 1>(),  make_t2u8<8, 1>(),  make_t2u8<9, 1>(),  make_t2u8<10, 1>(),
+    make_t2u8<11, 1>(), make_t2u8<12, 1>(), make_t2u8<1, 3>(),  make_t2u8<2, 3>(),  make_t2u8<3, 3>(),
+    make_t2u8<4, 3>(),  make_t2u8<5, 3>(),  make_t2u8<6, 3>(),  make_t2u8<7, 3>(),  make_t2u8<8, 3>(),
+    make_t2u8<9, 3>(),  make_t2u8<10, 3>(), make_t2u8<11, 3>(), make_t2u8<12, 3>(),
+};
+
 bool fits32t(int64_t v) { return v >= INT_MIN && v <= INT_MAX; }
 
 // cudaFuncSetAttribute once per kernel and device
@@ -243,21 +290,28 @@ itkg_status prepare_t2(const void* fn, size_t smem) {
 // The launch arguments of one request, its table entry and tile count;
 // ITKG_ERROR_UNSUPPORTED (no error set) when the tile kernel does not cover it.
 itkg_status build_t2(const FusedGeom& g, const float* const w[kMaxDim], Tile2DArgs* out, const EntryT2** entry,
-                     int64_t* ntiles) {
+                     int64_t* ntiles, bool u8 = false) {
   const bool slices = g.dim == 3 && g.radius[2] == 0 && w[2] && w[2][0] == 1.0f;
   if (g.u8pix) return ITKG_ERROR_UNSUPPORTED;
-  if ((g.dim != 2 && !slices) || g.in_dtype != ITKG_F32 || g.out_dtype == ITKG_I16) return ITKG_ERROR_UNSUPPORTED;
+  if ((g.dim != 2 && !slices) || g.in_dtype != (u8 ? ITKG_U8 : ITKG_F32) || g.out_dtype == ITKG_I16)
+    return ITKG_ERROR_UNSUPPORTED;
   if (g.radius[0] != g.radius[1] || g.radius[0] < 1) return ITKG_ERROR_UNSUPPORTED;
   const EntryT2* e = nullptr;
-  for (const EntryT2& t : kTableT2)
-    if (t.r == g.radius[0] && t.comps == g.comps) e = &t;
+  if (u8) {
+    for (const EntryT2& t : kTableT2U8)
+      if (t.r == g.radius[0] && t.comps == g.comps) e = &t;
+  } else {
+    for (const EntryT2& t : kTableT2)
+      if (t.r == g.radius[0] && t.comps == g.comps) e = &t;
+  }
   if (!e) return ITKG_ERROR_UNSUPPORTED;
   for (int d = 0; d < 2; ++d)
     if (!fits32t(g.lo[d]) || !fits32t(g.hi[d]) || !fits32t(g.src_origin[d]) || !fits32t(g.dst_origin[d]) ||
         !fits32t(g.req_index[d] + g.req_size[d] + kTH) || !fits32t(g.req_index[d] - 64))
       return ITKG_ERROR_UNSUPPORTED;
-  if (g.src_pitch[0] != 4 * g.comps || ((uintptr_t)g.src & 3) || (g.src_pitch[1] & 3) ||
-      (slices && (g.src_pitch[2] & 3)))
+  if (u8 ? g.src_pitch[0] != g.comps
+         : g.src_pitch[0] != 4 * g.comps || ((uintptr_t)g.src & 3) || (g.src_pitch[1] & 3) ||
+               (slices && (g.src_pitch[2] & 3)))
     return ITKG_ERROR_UNSUPPORTED;
   const int64_t nz = slices ? g.req_size[2] : 1;
   const int64_t ntx = (g.req_size[0] + kTW - 1) / kTW, nty = (g.req_size[1] + kTH - 1) / kTH;
@@ -294,12 +348,12 @@ itkg_status build_t2(const FusedGeom& g, const float* const w[kMaxDim], Tile2DAr
 
 }  // namespace
 
-itkg_status launch_tile2d(const FusedGeom& g, const float* const w[kMaxDim], void* stream, bool dry_run) {
+static itkg_status launch_t2(const FusedGeom& g, const float* const w[kMaxDim], void* stream, bool dry_run, bool u8) {
   Tile2DArgs a;
   const EntryT2* e = nullptr;
   int64_t ntiles = 0;
   {
-    const itkg_status st = build_t2(g, w, &a, &e, &ntiles);
+    const itkg_status st = build_t2(g, w, &a, &e, &ntiles, u8);
     if (st != ITKG_SUCCESS) return st;
   }
   if (dry_run) return ITKG_SUCCESS;
@@ -311,9 +365,17 @@ itkg_status launch_tile2d(const FusedGeom& g, const float* const w[kMaxDim], voi
   }
   fn<<<(unsigned)ntiles, kT2Threads, e->smem, static_cast<cudaStream_t>(stream)>>>(a);
   const cudaError_t err = cudaGetLastError();
-  note_launch(ref ? "tile2d_f32_ref" : "tile2d_f32_fma");
+  note_launch(u8 ? (ref ? "tile2d_u8_ref" : "tile2d_u8_fma") : (ref ? "tile2d_f32_ref" : "tile2d_f32_fma"));
   if (err != cudaSuccess) return set_error(ITKG_ERROR_CUDA, "tile2d launch: %s", cudaGetErrorString(err));
   return ITKG_SUCCESS;
+}
+
+itkg_status launch_tile2d(const FusedGeom& g, const float* const w[kMaxDim], void* stream, bool dry_run) {
+  return launch_t2(g, w, stream, dry_run, false);
+}
+
+itkg_status launch_tile2d_u8(const FusedGeom& g, const float* const w[kMaxDim], void* stream, bool dry_run) {
+  return launch_t2(g, w, stream, dry_run, true);
 }
 
 // Multi-request launches: the requests grouped by kernel class, one launch per
