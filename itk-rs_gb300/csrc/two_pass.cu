@@ -190,6 +190,17 @@ itkg_status launch_two_pass(const FusedGeom& g, const float* const w[kMaxDim], v
     e = find_xy(g.radius[0], g.in_dtype);
   }
   if (!e) return ITKG_ERROR_UNSUPPORTED;
+  // Tile height: 96 rows where they pad the image's height less than 128 do
+  // (192 rows: two tiles instead of 256 rows' work), counting a tile's x pass
+  // rows (its height and 2r) and y pass rows.  192 x ny x 192, radius 6, both
+  // tile heights, FMA / reference / u8 us: ny 96 20.1 and 16.6 / 27.5 and 22.7 /
+  // 27.1 and 21.8, ny 192 30.7 and 24.0 / 46.3 and 38.9 / 46.4 and 38.1.
+  if (g.radius[0] <= 8 && (u8p || g.in_dtype == ITKG_F32 || g.in_dtype == ITKG_I16)) {
+    const int64_t h = g.req_size[1], r = g.radius[0];
+    auto cost = [&](int64_t ty) { return (h + ty - 1) / ty * (2 * ty + 2 * r); };
+    if (cost(96) < cost(128))
+      e = (u8p ? twopass::xy96_u8p() : g.in_dtype == ITKG_F32 ? twopass::xy96_f32() : twopass::xy96_i16()) + (r - 1);
+  }
   const int esz = dtype_size(g.in_dtype);
   if (g.src_pitch[0] != esz) return ITKG_ERROR_UNSUPPORTED;
   // FMA rounding reads zeros outside the input buffer as the halo and adds the
@@ -354,7 +365,10 @@ itkg_status launch_two_pass(const FusedGeom& g, const float* const w[kMaxDim], v
     za.ush_pitch[2] = g.src_pitch[2];
   }
   for (int k = 0; k < 2 * rz + 1; ++k) za.wz[k] = w[2][k], za.wz2[k] = splat2_host(w[2][k]);
-  const int64_t qblocks = ntx * nty * (tile_floats / 4 / twopass::CfgZ<1>::QB);
+  // 32-row blocks (256 quads) that hold requested rows: blocks of a last tile's
+  // padding would unbalance the split (192 x 224 x 192, FMA: 31.0 us with them,
+  // 29.6 without)
+  const int64_t qblocks = ntx * ((ny + 31) / 32);
   za.tile_rows = e->ty;
 
   for (int64_t c0 = 0; c0 < nz && st == ITKG_SUCCESS; c0 += chunk) {

@@ -97,9 +97,9 @@ struct ZArgs {
   int32_t t_s0, t_s1;      // absolute z of T's first / last slice (the clamp bounds)
   int32_t nx, ny;          // requested columns / rows
   int32_t ntx;             // tiles along x
-  int32_t tile_rows;       // rows of a T tile (64 or 128)
+  int32_t tile_rows;       // rows of a T tile (64, 96 or 128)
   int32_t z0, nz;          // output slices of this launch (absolute) and count
-  int64_t units;           // quad blocks (256 quads each) * nz
+  int64_t units;           // quad blocks (32 rows of a tile column: 256 quads) * nz
   char* dst;               // output voxel (x0, y0, z0)
   int64_t dst_pitch[3];    // bytes
   int32_t out_dtype;
@@ -114,15 +114,16 @@ struct ZArgs {
   int32_t split[kMaxZSplit + 1];
 };
 
-template <int R, typename Tin>
+// TYV: the tile height for R <= 8 (128 or 96 rows; above, 64).
+template <int R, typename Tin, int TYV = 128>
 struct CfgXY {
   static constexpr int K = 2 * R + 1;
   static constexpr int ESZ = (int)sizeof(Tin);
   static constexpr int NT = 288;                // two x-pass tasks per thread (IH * SEGS <= 576)
   static constexpr int NTY = 256;               // threads of the y pass
   static constexpr int TX = kTileX;             // 16 lanes x 2 columns
-  static constexpr int MY = R <= 8 ? 8 : 4;     // rows per thread in the y pass
-  static constexpr int TY = (NTY / 16) * MY;    // 128 (64 for R > 8)
+  static constexpr int MY = R <= 8 ? TYV / 16 : 4;  // rows per thread in the y pass
+  static constexpr int TY = (NTY / 16) * MY;    // TYV (64 for R > 8)
   static constexpr int MX = 8;                  // x outputs per x-pass task
   static constexpr int SEGS = TX / MX;
   static constexpr int AE = 16 / ESZ;
@@ -160,7 +161,7 @@ struct CfgZ {
   static constexpr int QB = NT * QPT;           // quads per block of work
   static constexpr int S = KZ;                  // slices in flight per thread: one per phase
   static constexpr size_t SMEM = (size_t)S * NT * 16 * QPT;
-  static_assert((kTileX / 4 * 64) % QB == 0, "blocks of work tile the T tiles (64 or 128 rows)");
+  static_assert(kTileX / 4 * 32 == QB, "a block of work is 32 rows of a T tile (of 64, 96 or 128)");
 };
 
 // ---------------------------------------------------------------------------
@@ -232,11 +233,11 @@ __device__ __forceinline__ f2_t tap2_ref(f2_t acc, f2_t x, f2_t w, f2_t nz) { re
 // xy pass
 // U8P (with REF and u8 input): u8 pixel arithmetic; the weights are the
 // per-tap constants c, and T holds each y-pass output byte as an f32.
-template <int R, bool REF, typename Tin, bool U8P = false>
-__global__ void __launch_bounds__(288, CfgXY<R, Tin>::MINB)
+template <int R, bool REF, typename Tin, bool U8P = false, int TYV = 128>
+__global__ void __launch_bounds__(288, CfgXY<R, Tin, TYV>::MINB)
     k_xy_pass(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ XYArgs a) {
   static_assert(!U8P || (REF && std::is_same<Tin, uint8_t>::value), "u8 pixel arithmetic: clamped u8 tiles");
-  using C = CfgXY<R, Tin>;
+  using C = CfgXY<R, Tin, TYV>;
   constexpr int K = C::K, TX = C::TX, TY = C::TY, MY = C::MY, MX = C::MX, BW = C::BW, IH = C::IH,
                 XA = C::XA, S = C::S, WIN = C::WIN, WB = C::WB, OFF = C::OFF, NT = C::NT, SEGS = C::SEGS,
                 TXP = C::TXP, NTASK = C::NTASK, NXB = C::NXB;
@@ -573,14 +574,16 @@ __global__ void __launch_bounds__(256, RZ <= (REF ? 6 : 8) ? 2 : 1) k_z_pass(con
     const int64_t zrem = zs + (u_end - u);
     const int ze = zrem < a.nz ? (int)zrem : a.nz;
     u += ze - zs;
-    // this thread's quad: T tile `tl`, quad w (row w / 8, columns 4 (w % 8) .. + 3)
-    const int64_t q = blk * C::QB + tid;
+    // block: rows 32 rb .. + 31 of tile column tix (rows below the request have
+    // no block); this thread's quad: T tile `tl`, quad w (row w / 8, columns
+    // 4 (w % 8) .. + 3)
+    const int rb = (int)(blk / a.ntx), tix = (int)(blk - (int64_t)rb * a.ntx);
+    const int bpt = a.tile_rows / 32, tly = rb / bpt;
     const int tile_q = a.tile_rows * (kTileX / 4);  // quads per tile
-    const int64_t tl = q / tile_q;
-    const int w = (int)(q - tl * tile_q);
-    const int64_t tly = tl / a.ntx;
-    const int cx = (int)(tl - tly * a.ntx) * kTileX + 4 * (w & (kTileX / 4 - 1));  // first column
-    const int cy = (int)tly * a.tile_rows + w / (kTileX / 4);                      // row
+    const int64_t tl = (int64_t)tly * a.ntx + tix;
+    const int w = (rb - tly * bpt) * C::QB + tid;
+    const int cx = tix * kTileX + 4 * (w & (kTileX / 4 - 1));     // first column
+    const int cy = tly * a.tile_rows + w / (kTileX / 4);          // row
     if (cy >= a.ny || cx >= a.nx) continue;  // no barriers in this kernel: idle threads just skip
     const int z0 = a.z0 + zs, z1 = a.z0 + ze;  // outputs [z0, z1)
     const int jb = z0 - RZ;
@@ -753,11 +756,11 @@ struct XYEntry {
   int tx, ty, bw, ih;  // tile, TMA box
 };
 
-template <int R, typename Tin>
+template <int R, typename Tin, int TYV = 128>
 XYEntry make_xy(int dtype) {
-  using C = CfgXY<R, Tin>;
-  return XYEntry{R, dtype, {k_xy_pass<R, false, Tin>, k_xy_pass<R, true, Tin>}, C::SMEM, C::NT, C::TX, C::TY, C::BW,
-                 C::IH};
+  using C = CfgXY<R, Tin, TYV>;
+  return XYEntry{R, dtype, {k_xy_pass<R, false, Tin, false, TYV>, k_xy_pass<R, true, Tin, false, TYV>}, C::SMEM, C::NT,
+                 C::TX, C::TY, C::BW, C::IH};
 }
 
 // Tables: two_pass.cu (f32 x-y), two_pass_in.cu (i16, u8, bf16, f16 x-y), two_pass_z*.cu (z).
@@ -766,6 +769,11 @@ const XYEntry* xy_entries_i16(int* n);
 const XYEntry* xy_entries_u8(int* n);
 const XYEntry* xy_entries_bf16(int* n);
 const XYEntry* xy_entries_f16(int* n);
+// The same with 96-row tiles, radii 1 .. 8: f32 and i16 (two_pass_xy96.cu), u8
+// pixel arithmetic (two_pass_u8p.cu); [r - 1].
+const XYEntry* xy96_f32();
+const XYEntry* xy96_i16();
+const XYEntry* xy96_u8p();
 ZFn z_fn(int r, bool ref, int store, bool ush = false);
 // The plain z kernels, split over translation units so they compile in
 // parallel: [r - 1] of each row is k_z_pass<r, REF, ST>.

@@ -6,16 +6,20 @@
 namespace itkg {
 namespace twopass {
 namespace {
-template <int R>
+template <int R, int TYV = 128>
 XYEntry make_xy_u8p() {
-  using C = CfgXY<R, uint8_t>;
-  const XYFn f = k_xy_pass<R, true, uint8_t, true>;
+  using C = CfgXY<R, uint8_t, TYV>;
+  const XYFn f = k_xy_pass<R, true, uint8_t, true, TYV>;
   return XYEntry{R, ITKG_U8, {f, f}, C::SMEM, C::NT, C::TX, C::TY, C::BW, C::IH};
 }
 const XYEntry kXYU8P[] = {make_xy_u8p<1>(), make_xy_u8p<2>(),  make_xy_u8p<3>(),  make_xy_u8p<4>(),
                           make_xy_u8p<5>(), make_xy_u8p<6>(),  make_xy_u8p<7>(),  make_xy_u8p<8>(),
                           make_xy_u8p<9>(), make_xy_u8p<10>(), make_xy_u8p<11>(), make_xy_u8p<12>()};
+const XYEntry kXYU8P96[] = {make_xy_u8p<1, 96>(), make_xy_u8p<2, 96>(), make_xy_u8p<3, 96>(), make_xy_u8p<4, 96>(),
+                            make_xy_u8p<5, 96>(), make_xy_u8p<6, 96>(), make_xy_u8p<7, 96>(), make_xy_u8p<8, 96>()};
 }  // namespace
+
+const XYEntry* xy96_u8p() { return kXYU8P96; }
 
 #define ITKG_Z_U8P_ROW(ST)                                                                            \
   {                                                                                                   \
