@@ -190,16 +190,25 @@ itkg_status launch_two_pass(const FusedGeom& g, const float* const w[kMaxDim], v
     e = find_xy(g.radius[0], g.in_dtype);
   }
   if (!e) return ITKG_ERROR_UNSUPPORTED;
-  // Tile height: 96 rows where they pad the image's height less than 128 do
-  // (192 rows: two tiles instead of 256 rows' work), counting a tile's x pass
-  // rows (its height and 2r) and y pass rows.  192 x ny x 192, radius 6, both
-  // tile heights, FMA / reference / u8 us: ny 96 20.1 and 16.6 / 27.5 and 22.7 /
-  // 27.1 and 21.8, ny 192 30.7 and 24.0 / 46.3 and 38.9 / 46.4 and 38.1.
+  // Tile height: 64 rows where one tile of them holds the image, else 96 or 128,
+  // whichever costs less: per tile its x pass rows (its height and 2r), its y
+  // pass rows, and a fixed part worth `fixed` rows (a row costs less at a small
+  // radius and in FMA rounding).  192 x ny x 192, radius 6, at 128 rows and at
+  // 96, FMA / reference / u8 us: ny 96 20.1 and 16.6 / 27.5 and 22.7 / 27.1 and
+  // 21.8, ny 192 30.7 and 24.0 / 46.3 and 38.9 / 46.4 and 38.1.  At 96 and at 64,
+  // 192 x 64 x 128: 12.1 and 11.8 / 17.4 and 15.2 / 17.3 and 15.1; more tiles of
+  // 64 rows than one gain 3 % at best (ny 320, radius 6) and lose 5 (radius 2).
+  // The fixed part: 192 x 430 x 128, radius 2, FMA: 4 tiles of 128 rows 34.5 us,
+  // 5 of 96 37.1.
   if (g.radius[0] <= 8 && (u8p || g.in_dtype == ITKG_F32 || g.in_dtype == ITKG_I16)) {
     const int64_t h = g.req_size[1], r = g.radius[0];
-    auto cost = [&](int64_t ty) { return (h + ty - 1) / ty * (2 * ty + 2 * r); };
-    if (cost(96) < cost(128))
-      e = (u8p ? twopass::xy96_u8p() : g.in_dtype == ITKG_F32 ? twopass::xy96_f32() : twopass::xy96_i16()) + (r - 1);
+    const int64_t fixed = (u8p || g.rounding == ITKG_ROUND_REFERENCE ? 128 : 256) / (r + 1);
+    auto cost = [&](int64_t ty) { return (h + ty - 1) / ty * (2 * ty + 2 * r + fixed); };
+    const int rows = h <= 64 ? 64 : cost(96) < cost(128) ? 96 : 128;
+    if (rows != 128)
+      e = (u8p                        ? twopass::xy_rows_u8p(rows)
+           : g.in_dtype == ITKG_F32 ? twopass::xy_rows_f32(rows)
+                                    : twopass::xy_rows_i16(rows)) + (r - 1);
   }
   const int esz = dtype_size(g.in_dtype);
   if (g.src_pitch[0] != esz) return ITKG_ERROR_UNSUPPORTED;

@@ -114,7 +114,7 @@ struct ZArgs {
   int32_t split[kMaxZSplit + 1];
 };
 
-// TYV: the tile height for R <= 8 (128 or 96 rows; above, 64).
+// TYV: the tile height for R <= 8 (128, 96 or 64 rows; above, 64).
 template <int R, typename Tin, int TYV = 128>
 struct CfgXY {
   static constexpr int K = 2 * R + 1;
@@ -149,7 +149,7 @@ struct CfgXY {
   static constexpr size_t SMEM = (size_t)S * STAGE + sizeof(float) * NXB * XBUF + 128;
   static_assert(WB + TX - MX + WIN <= BW, "x window stays inside the staged row");
   static_assert(TX % MX == 0, "x segments");
-  static_assert(NTASK > NT && NTASK <= 2 * NT, "each thread runs one or two x-pass tasks");
+  static_assert(NTASK <= 2 * NT, "each thread runs at most two x-pass tasks");
   static_assert(TY <= kTileY, "tile height");
 };
 
@@ -271,10 +271,10 @@ __global__ void __launch_bounds__(288, CfgXY<R, Tin, TYV>::MINB)
   const uint64_t pol_in = policy_evict_first();
   const uint64_t pol_t = policy_evict_last();
 
-  // this thread's x-pass tasks: (row, 8-column segment) tid and tid + NT (if < NTASK)
+  // this thread's x-pass tasks: (row, 8-column segment) tid and tid + NT (where < NTASK)
   const int row_a = tid / SEGS, x0_a = (tid % SEGS) * MX;
   const int row_b = (tid + NT) / SEGS, x0_b = ((tid + NT) % SEGS) * MX;
-  const bool has_b = tid + NT < NTASK;
+  const bool has_a = NTASK >= NT || tid < NTASK, has_b = tid + NT < NTASK;
   // this thread's y-pass share: columns 2*lane16, +1; rows grp*MY .. +MY-1
   const int lane16 = tid & 15, grp = tid >> 4;
   const bool has_y = tid < C::NTY;
@@ -420,7 +420,7 @@ __global__ void __launch_bounds__(288, CfgXY<R, Tin, TYV>::MINB)
       phase_bits ^= 1u << st_use;
       st_use = st_use + 1 == S ? 0 : st_use + 1;
       ++n_consumed;
-      xtask(tile_s, xb, row_a, x0_a, yedge, rlo, rhi, xedge, nl, cr);
+      if (has_a) xtask(tile_s, xb, row_a, x0_a, yedge, rlo, rhi, xedge, nl, cr);
       if (has_b) xtask(tile_s, xb, row_b, x0_b, yedge, rlo, rhi, xedge, nl, cr);
     };
 
@@ -769,11 +769,11 @@ const XYEntry* xy_entries_i16(int* n);
 const XYEntry* xy_entries_u8(int* n);
 const XYEntry* xy_entries_bf16(int* n);
 const XYEntry* xy_entries_f16(int* n);
-// The same with 96-row tiles, radii 1 .. 8: f32 and i16 (two_pass_xy96.cu), u8
-// pixel arithmetic (two_pass_u8p.cu); [r - 1].
-const XYEntry* xy96_f32();
-const XYEntry* xy96_i16();
-const XYEntry* xy96_u8p();
+// The same with 96- and 64-row tiles, radii 1 .. 8: f32 and i16
+// (two_pass_xyrows.cu), u8 pixel arithmetic (two_pass_u8p.cu); [r - 1].
+const XYEntry* xy_rows_f32(int rows);
+const XYEntry* xy_rows_i16(int rows);
+const XYEntry* xy_rows_u8p(int rows);
 ZFn z_fn(int r, bool ref, int store, bool ush = false);
 // The plain z kernels, split over translation units so they compile in
 // parallel: [r - 1] of each row is k_z_pass<r, REF, ST>.

@@ -15,11 +15,15 @@ XYEntry make_xy_u8p() {
 const XYEntry kXYU8P[] = {make_xy_u8p<1>(), make_xy_u8p<2>(),  make_xy_u8p<3>(),  make_xy_u8p<4>(),
                           make_xy_u8p<5>(), make_xy_u8p<6>(),  make_xy_u8p<7>(),  make_xy_u8p<8>(),
                           make_xy_u8p<9>(), make_xy_u8p<10>(), make_xy_u8p<11>(), make_xy_u8p<12>()};
-const XYEntry kXYU8P96[] = {make_xy_u8p<1, 96>(), make_xy_u8p<2, 96>(), make_xy_u8p<3, 96>(), make_xy_u8p<4, 96>(),
-                            make_xy_u8p<5, 96>(), make_xy_u8p<6, 96>(), make_xy_u8p<7, 96>(), make_xy_u8p<8, 96>()};
+#define ITKG_XY_U8P_ROWS(TY)                                                                   \
+  {                                                                                            \
+    make_xy_u8p<1, TY>(), make_xy_u8p<2, TY>(), make_xy_u8p<3, TY>(), make_xy_u8p<4, TY>(),     \
+        make_xy_u8p<5, TY>(), make_xy_u8p<6, TY>(), make_xy_u8p<7, TY>(), make_xy_u8p<8, TY>()  \
+  }
+const XYEntry kXYU8PRows[2][8] = {ITKG_XY_U8P_ROWS(96), ITKG_XY_U8P_ROWS(64)};
 }  // namespace
 
-const XYEntry* xy96_u8p() { return kXYU8P96; }
+const XYEntry* xy_rows_u8p(int rows) { return kXYU8PRows[rows == 64]; }
 
 #define ITKG_Z_U8P_ROW(ST)                                                                            \
   {                                                                                                   \

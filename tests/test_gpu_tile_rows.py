@@ -1,8 +1,8 @@
 """Tile heights of the two-pass forward's x-y kernel: heights on both sides of
-where 96-row tiles take over from 128-row ones, several tiles high and with last
-tiles of a few rows, at radii with either tile (<= 8) and with 64 rows (9); the
-i16 and u8 forms too.  Reference rounding and u8 pixel arithmetic are bit-exact,
-fused multiply-adds within their rounding."""
+where 64-, 96- and 128-row tiles take over from each other, several tiles high
+and with last tiles of a few rows, at radii with any of them (<= 8) and with 64
+rows (9); the i16 and u8 forms too.  Reference rounding and u8 pixel arithmetic
+are bit-exact, fused multiply-adds within their rounding."""
 import numpy as np
 import pytest
 
@@ -11,8 +11,8 @@ import oracle
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("ny", [1, 31, 95, 96, 97, 128, 129, 192, 193, 257, 288])
-@pytest.mark.parametrize("radius", [1, 6, 8, 9])
+@pytest.mark.parametrize("ny", [1, 31, 63, 64, 65, 95, 96, 97, 128, 129, 192, 193, 257, 288, 320])
+@pytest.mark.parametrize("radius", [1, 3, 4, 6, 8, 9])
 def test_heights(gpu, ny, radius):
     sigma = radius / 3.0
     shape = (radius + 2, ny, 41)
@@ -33,8 +33,8 @@ def test_heights(gpu, ny, radius):
                 assert np.abs(got - want).max() <= 6 * (2 * radius + 2) * 2.0 ** -24 * np.abs(xf).max()
 
 
-@pytest.mark.parametrize("ny", [31, 96, 97, 192, 257])
-@pytest.mark.parametrize("radius", [1, 6, 8, 9])
+@pytest.mark.parametrize("ny", [31, 64, 96, 97, 192, 257, 320])
+@pytest.mark.parametrize("radius", [1, 3, 4, 6, 8, 9])
 def test_u8_heights(gpu, ny, radius):
     sigma = radius / 3.0
     x = np.random.default_rng(ny + radius).integers(0, 256, (radius + 2, ny, 41), dtype=np.uint8)
