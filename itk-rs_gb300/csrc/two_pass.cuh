@@ -574,14 +574,17 @@ __global__ void __launch_bounds__(256, RZ <= (REF ? 6 : 8) ? 2 : 1) k_z_pass(con
     const int64_t zrem = zs + (u_end - u);
     const int ze = zrem < a.nz ? (int)zrem : a.nz;
     u += ze - zs;
-    // block: rows 32 rb .. + 31 of tile column tix (rows below the request have
-    // no block); this thread's quad: T tile `tl`, quad w (row w / 8, columns
-    // 4 (w % 8) .. + 3)
-    const int rb = (int)(blk / a.ntx), tix = (int)(blk - (int64_t)rb * a.ntx);
-    const int bpt = a.tile_rows / 32, tly = rb / bpt;
+    // block: 32 rows of tile (tix, tly), the blocks of a tile one after another as
+    // the x-y pass walks its tiles, so that a CTA reads T about where the x-y CTA
+    // of the same number wrote it (rows below the request have no block); this
+    // thread's quad: T tile `tl`, quad w (row w / 8, columns 4 (w % 8) .. + 3)
+    const int bpt = a.tile_rows / 32, nrb = (a.ny + 31) / 32;
+    const int tly = (int)blk / (a.ntx * bpt), in_row = (int)blk - tly * a.ntx * bpt;
+    const int nb = min(bpt, nrb - tly * bpt);  // blocks of this row's tiles
+    const int tix = in_row / nb;
     const int tile_q = a.tile_rows * (kTileX / 4);  // quads per tile
     const int64_t tl = (int64_t)tly * a.ntx + tix;
-    const int w = (rb - tly * bpt) * C::QB + tid;
+    const int w = (in_row - tix * nb) * C::QB + tid;
     const int cx = tix * kTileX + 4 * (w & (kTileX / 4 - 1));     // first column
     const int cy = tly * a.tile_rows + w / (kTileX / 4);          // row
     if (cy >= a.ny || cx >= a.nx) continue;  // no barriers in this kernel: idle threads just skip
