@@ -189,15 +189,39 @@ DotArgs dot_args(const itkg_image& p, const itkg_image& q) {
   return d;
 }
 
-// Reads n doubles from the device after the work queued on s, through a pinned
-// buffer of the calling thread (a copy to pageable memory is staged by the
-// driver and cost a single result 8 us more).  Synchronises s.
+// A pinned buffer of the calling thread, freed with it.  Allocating pinned memory
+// is not allowed while another thread captures a graph in the global mode, and
+// would end that capture; the relaxed mode of this thread lifts that (the
+// allocation belongs to no graph).
 constexpr int kPinnedDoubles = 64;
+struct PinnedDoubles {
+  double* p = nullptr;
+  double* get() {
+    if (!p) {
+      cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+      if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) return nullptr;
+      if (cudaMallocHost(reinterpret_cast<void**>(&p), sizeof(double) * kPinnedDoubles) != cudaSuccess) {
+        cudaGetLastError();
+        p = nullptr;
+      }
+      cudaThreadExchangeStreamCaptureMode(&mode);
+    }
+    return p;
+  }
+  ~PinnedDoubles() {
+    if (!p) return;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    if (cudaThreadExchangeStreamCaptureMode(&mode) == cudaSuccess) cudaFreeHost(p);
+  }
+};
+
+// Reads n doubles from the device after the work queued on s, through a pinned
+// buffer where there is one (a copy to pageable memory is staged by the driver
+// and cost a single result 8 us more).  Synchronises s.
 itkg_status read_back(const double* dev, int n, double* out, cudaStream_t s) {
-  thread_local double* pinned = nullptr;
-  if (n <= kPinnedDoubles && !pinned)
-    ITKG_CUDA(cudaMallocHost(reinterpret_cast<void**>(&pinned), sizeof(double) * kPinnedDoubles));
-  double* const to = n <= kPinnedDoubles ? pinned : out;
+  thread_local PinnedDoubles pinned;
+  double* to = n <= kPinnedDoubles ? pinned.get() : nullptr;
+  if (!to) to = out;
   ITKG_CUDA(cudaMemcpyAsync(to, dev, sizeof(double) * (size_t)n, cudaMemcpyDeviceToHost, s));
   ITKG_CUDA(cudaStreamSynchronize(s));
   if (to != out) std::memcpy(out, to, sizeof(double) * (size_t)n);
