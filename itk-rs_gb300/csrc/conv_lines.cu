@@ -9,7 +9,9 @@
 // order from zero exactly as the one-output-per-thread pass does, bit for bit
 // in either rounding.  Inputs and taps beyond an output's window are never
 // multiplied in (the first and last M - 1 inputs run as unrolled triangles),
-// so an infinity or NaN reaches the same outputs as before.  The M live taps
+// so an infinity or NaN reaches the same outputs as before.  The inputs of a
+// run that ends past the request are clamped to the request's last tap
+// (line_window.hpp): a pass's source ends there.  The M live taps
 // sit in registers and shift by one per input.
 //
 //   k_lines_yz  passes along y and z: lanes on columns c and c + 32 of a
@@ -40,12 +42,13 @@
 
 #include "f32x2.cuh"
 #include "internal.hpp"
+#include "line_window.hpp"
 #include "pixel.cuh"
 
 namespace itkg {
 namespace {
 
-constexpr int kM = 16;         // outputs per thread
+constexpr int kM = kLineRun;   // outputs per thread
 constexpr int kStrip = 64;     // lines per warp (two per lane)
 constexpr int kRowPitch = 66;  // k_lines_x: floats per staged x position
 constexpr int kMaxWarps = 8;
@@ -148,20 +151,18 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 2) k_lines_yz(const __grid_con
   const int64_t left = (md == 1 ? a.out_size[1] : a.out_size[2]) - (int64_t)run * kM;
   const int nv = (int)(left < kM ? left : kM);
   const f2_t nz = pack2(p.nz, p.nz);
-  // the window's first position and the last one of the image, from the image's first
-  const int first = (int)(m_at - a.radius - a.lo), last = (int)(a.hi - a.lo);
+  const LineWindow win = line_window(m_at, nv, a.radius, a.lo, a.hi);
   const int64_t dmp = md == 1 ? a.dst_pitch[1] : a.dst_pitch[2], dop = od == 1 ? a.dst_pitch[1] : a.dst_pitch[2];
   const int64_t dmo = md == 1 ? a.dst_origin[1] : a.dst_origin[2], doo = od == 1 ? a.dst_origin[1] : a.dst_origin[2];
   for (int64_t o = blockIdx.z; o < on; o += gridDim.z) {
-    // a pointer that steps by one pitch while the next position is inside the image
+    // a pointer that steps by one pitch from window entry to window entry
     const char* s = static_cast<const char*>(a.src) + (a.out_index[0] - a.src_origin[0]) * a.src_pitch[0] + c0 * 4 +
-                    (o_first + o - oo) * op + (a.lo - mo + min(max(first, 0), last)) * mp;
+                    (o_first + o - oo) * op + (a.lo - mo + line_at(win, 0)) * mp;
     f2_t acc[kM];
     walk<REF>(W.w2, a.radius, nz, acc, [&](int j) {
       const float* const f = reinterpret_cast<const float*>(s);
       const f2_t v = pack2(__ldg(f), __ldg(f + d1));
-      // position first + j + 1, clamped, is one further only while in 1 .. last
-      s += (unsigned)(first + j) < (unsigned)last ? mp : 0;
+      s += line_steps(win, j) ? mp : 0;
       return v;
     });
     char* d = static_cast<char*>(a.dst) + (a.out_index[0] - a.dst_origin[0]) * a.dst_pitch[0] +
@@ -195,8 +196,8 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 2) k_lines_x(const __grid_cons
   const int x_first = blockIdx.x * nw * kM;  // first output of the block
   const int64_t x_left = a.out_size[0] - x_first;
   const int span = (int)min((int64_t)nw * kM, x_left);  // outputs of the block inside the request
-  const int width = nw * kM + 2 * a.radius;              // staged positions (clamped to the image)
-  const int first = (int)(a.out_index[0] + x_first - a.radius - a.lo), last = (int)(a.hi - a.lo);
+  const int width = nw * kM + 2 * a.radius;              // staged positions
+  const LineWindow win = line_window(a.out_index[0] + x_first, span, a.radius, a.lo, a.hi);
   const f2_t nz = pack2(p.nz, p.nz);
   __shared__ int64_t s_src[kStrip], s_dst[kStrip];  // byte offsets of the group's lines
   const char* const src = static_cast<const char*>(a.src) + (a.lo - a.src_origin[0]) * a.src_pitch[0];
@@ -213,8 +214,8 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 2) k_lines_x(const __grid_cons
     }
     __syncthreads();
     // stage: warp w takes line pairs 2w, 2w + 1, then 2 (w + nw), ...; lanes
-    // along x, four positions each: 16 loads in flight per thread (positions
-    // past the tile are read, clamped, and dropped)
+    // along x, four positions each: 16 loads in flight per thread (entries
+    // past the tile repeat the window's last position and are dropped)
     static_assert(kStrip / 2 % 2 == 0, "whole quads of lines");
     for (int pr = 2 * warp; pr < kStrip / 2; pr += 2 * nw) {
       const char* sl[4];
@@ -225,7 +226,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 2) k_lines_x(const __grid_cons
         float v[4][4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-          const int64_t off = (int64_t)min(max(first + xb + 32 * q, 0), last) * a.src_pitch[0];
+          const int64_t off = (int64_t)line_at(win, xb + 32 * q) * a.src_pitch[0];
 #pragma unroll
           for (int i = 0; i < 4; ++i) v[q][i] = to_f32(*reinterpret_cast<const Tin*>(sl[i] + off));
         }
