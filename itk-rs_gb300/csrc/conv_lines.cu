@@ -161,7 +161,10 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 2) k_lines_yz(const __grid_con
     f2_t acc[kM];
     walk<REF>(W.w2, a.radius, nz, acc, [&](int j) {
       const float* const f = reinterpret_cast<const float*>(s);
-      const f2_t v = pack2(__ldg(f), __ldg(f + d1));
+      // (plain loads: the previous pass may write this memory while this block
+      // waits in pdl_begin, and read-only loads ask for memory that nothing
+      // writes during the kernel)
+      const f2_t v = pack2(f[0], f[d1]);
       s += line_steps(win, j) ? mp : 0;
       return v;
     });

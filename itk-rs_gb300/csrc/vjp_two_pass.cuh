@@ -291,11 +291,12 @@ __global__ void __launch_bounds__(256, 2)
                               (int64_t)(sl - a.lo[2]) * a.u_pitch[2];
           const float* const ud = reinterpret_cast<const float*>(a.u + off);
           const float* const uv = reinterpret_cast<const float*>(a.u2 + off);
-          pu[m][0] = __ldg(ud);
-          pu2[m][0] = __ldg(uv);
+          // (plain loads: the z adjoint may write U and U' while this block waits in pdl_begin)
+          pu[m][0] = ud[0];
+          pu2[m][0] = uv[0];
           if (c1ok) {
-            pu[m][1] = __ldg(ud + 1);
-            pu2[m][1] = __ldg(uv + 1);
+            pu[m][1] = ud[1];
+            pu2[m][1] = uv[1];
           }
         }
       }
