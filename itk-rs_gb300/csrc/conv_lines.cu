@@ -39,6 +39,9 @@
 #include <algorithm>
 #include <cstdint>
 #include <cstring>
+#include <mutex>
+#include <utility>
+#include <vector>
 
 #include "f32x2.cuh"
 #include "internal.hpp"
@@ -286,6 +289,32 @@ int warps_for(int64_t runs, int most) {
   return (int)((runs + blocks - 1) / blocks);
 }
 
+// k_lines_x's dynamic shared memory for nw warps at radius R, and the most it
+// takes.  Beside it the kernel has 1 KB of its own (line offsets), which counts
+// against the 48 KB that need no opt-in.
+constexpr size_t x_smem(int nw, int R) { return (size_t)(nw * kM + 2 * R) * kRowPitch * sizeof(float); }
+constexpr int kMaxR = (kMaxParamTaps - 1) / 2;
+constexpr size_t kXSmemMost = std::max(x_smem(kMaxWarps, kBigR), x_smem(kWarps, kMaxR));
+static_assert(kXSmemMost + 2 * kStrip * sizeof(int64_t) <= 227 * 1024, "k_lines_x fits a block");
+
+// The limit on dynamic shared memory is the kernel's, shared by every thread
+// that launches it: set once per kernel and device, to the most that any call
+// takes, so that no call lowers it under another's launch.
+std::mutex g_x_mu;
+std::vector<std::pair<const void*, int>> g_x_ready;
+itkg_status prepare_x(const void* fn) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return set_error(ITKG_ERROR_CUDA, "cudaGetDevice: %s", cudaGetErrorString(e));
+  std::lock_guard<std::mutex> lk(g_x_mu);
+  for (const auto& r : g_x_ready)
+    if (r.first == fn && r.second == dev) return ITKG_SUCCESS;
+  e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kXSmemMost);
+  if (e != cudaSuccess) return set_error(ITKG_ERROR_CUDA, "conv_lines smem: %s", cudaGetErrorString(e));
+  g_x_ready.push_back({fn, dev});
+  return ITKG_SUCCESS;
+}
+
 }  // namespace
 
 itkg_status launch_conv_lines(const AxisArgs& a, const float* w, int in_dtype, int out_dtype, int rounding,
@@ -320,12 +349,9 @@ itkg_status launch_conv_lines(const AxisArgs& a, const float* w, int in_dtype, i
     const int64_t groups = (a.out_size[1] * a.out_size[2] * a.comps + kStrip - 1) / kStrip;
     block = dim3(32, (unsigned)nw);
     grid = dim3((unsigned)((p.runs + nw - 1) / nw), (unsigned)std::min<int64_t>(groups, 65535));
-    smem = (size_t)(nw * kM + 2 * a.radius) * kRowPitch * sizeof(float);
-    if (smem > 48 * 1024) {
-      const cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(fn),
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) return set_error(ITKG_ERROR_CUDA, "conv_lines smem: %s", cudaGetErrorString(e));
-    }
+    smem = x_smem(nw, a.radius);
+    const itkg_status st = prepare_x(reinterpret_cast<const void*>(fn));
+    if (st != ITKG_SUCCESS) return st;
   } else {
     if (in_dtype != ITKG_F32) return ITKG_ERROR_UNSUPPORTED;
     const bool full = a.out_size[0] * a.comps >= kStrip;
