@@ -60,10 +60,11 @@ __global__ void __launch_bounds__(kT) k_unsharp(const char* in, int64_t ip0, int
 
 // Scalar f32 rows of 16-byte aligned quads (x pitch 4, 16-byte aligned rows; the
 // last quad of a row may be ragged): thread i of the grid takes quads i, i +
-// grid, ... of the rows x quads space, streaming loads and stores.  The blur may
-// be the output image itself: a thread reads its quads before it writes them,
-// and a deferred voxel keeps its blur until k_unsharp_deferred replaces it.  I: the index type
-// (32-bit when the voxel count allows, for cheaper divisions).
+// grid, ... of the rows x quads space, streaming loads and stores.  The blur or
+// the input may be the output image itself: a thread reads its quads before it
+// writes them, and a deferred voxel keeps what k_unsharp_deferred will read
+// there (the blur where the output holds it, else the original).  I: the index
+// type (32-bit when the voxel count allows, for cheaper divisions).
 //
 // Voxels the f32 test cannot decide (a few in a thousand on smooth data) are
 // not computed in place: in f64 a warp would stall on every one of them.  The
@@ -147,7 +148,7 @@ __global__ void __launch_bounds__(kQT) k_unsharp_quads(const char* in, int64_t i
           const uint32_t slot = defer ? atomicAdd(&n_def, 1u) : kDeferCap;
           if (slot < kDeferCap) {
             seg[slot] = i * 4 + (I)c;
-            r[c] = bv[c];  // replaced by k_unsharp_deferred
+            r[c] = blur == out ? bv[c] : ov[c];  // replaced by k_unsharp_deferred
           } else {
             r[c] = __double2float_rn(unsharp_f64((double)ov[c], (double)bv[c], k.amount, k.threshold));
           }
