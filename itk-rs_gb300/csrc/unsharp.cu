@@ -62,29 +62,15 @@ __global__ void __launch_bounds__(kT) k_unsharp(const char* in, int64_t ip0, int
 // last quad of a row may be ragged): thread i of the grid takes quads i, i +
 // grid, ... of the rows x quads space, streaming loads and stores.  The blur or
 // the input may be the output image itself: a thread reads its quads before it
-// writes them, and a deferred voxel keeps what k_unsharp_deferred will read
-// there (the blur where the output holds it, else the original).  I: the index
-// type (32-bit when the voxel count allows, for cheaper divisions).
+// writes them.  I: the index type (32-bit when the voxel count allows, for
+// cheaper divisions).
 //
-// Voxels the f32 test cannot decide (a few in a thousand on smooth data) are
-// not computed in place: in f64 a warp would stall on every one of them.  The
-// block appends (quad index * 4 + lane) to its own segment of `defer`
-// (kDeferCap entries; its count in defer_n[block]) and k_unsharp_deferred
-// finishes them afterwards, a handful of f64 sequences per block.  Entries
-// past the segment's capacity are computed in place, and so are all with
-// defer NULL (FMA rounding and amounts that are f32: the f32 rules leave next
-// to none open).
+// Voxels the f32 rules cannot decide (a few in 10^5) take the f64 sequence in
+// place.  Collecting them for a second kernel was slower at every size: amount
+// 0.37, smooth / white data, the call: 61^3 19.7 / 19.5 us with a list, 16.9 /
+// 14.9 in place; 193 x 194 x 195 84.8 / 79.6 and 83.1 / 74.9; 255^2 14.5 / 14.5
+// and 10.4 / 10.3; 2047 x 2049 45.4 / 43.5 and 45.0 / 39.1.
 constexpr int kQT = 256;
-constexpr int kDeferCap = 2048;
-
-template <typename I>
-__device__ __forceinline__ void quad_addr(I i, I nq, I m1, int64_t p1, int64_t p2, int64_t& off, I& qx) {
-  const I row = i / nq;
-  qx = i - row * nq;
-  const I z = row / m1;
-  const I y = row - z * m1;
-  off = (int64_t)y * p1 + (int64_t)z * p2;
-}
 
 // The first n (< 4) floats of a quad, zeros after them.
 __device__ __forceinline__ float4 load_ragged(const float* p, int n) {
@@ -94,16 +80,11 @@ __device__ __forceinline__ float4 load_ragged(const float* p, int n) {
 template <typename I>
 __global__ void __launch_bounds__(kQT) k_unsharp_quads(const char* in, int64_t ip1, int64_t ip2, const char* blur,
                                                         int64_t bp1, int64_t bp2, char* out, int64_t op1, int64_t op2,
-                                                        I nq, I m0, I m1, I total, const UnsharpConsts k, I* defer,
-                                                        uint32_t* defer_n) {
-  __shared__ uint32_t n_def;
-  if (threadIdx.x == 0) n_def = 0;
-  __syncthreads();
+                                                        I nq, I m0, I m1, I total, const UnsharpConsts k) {
   // a programmatic dependent of the blur's last kernel, and the next call's
   // first kernel may be one of this: each waits before it touches memory
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
   asm volatile("griddepcontrol.wait;\n" ::: "memory");
-  I* const seg = defer + (size_t)blockIdx.x * kDeferCap;
   // two quads per step (i and i + stride), their loads issued together
   const I stride = (I)gridDim.x * kQT;
   for (I i0 = (I)blockIdx.x * kQT + threadIdx.x; i0 < total; i0 += 2 * stride) {
@@ -137,7 +118,6 @@ __global__ void __launch_bounds__(kQT) k_unsharp_quads(const char* in, int64_t i
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       if (!live[h]) continue;
-      const I i = i0 + (I)h * stride;
       const float ov[4] = {o[h].x, o[h].y, o[h].z, o[h].w}, bv[4] = {b[h].x, b[h].y, b[h].z, b[h].w};
       float r[4];
 #pragma unroll
@@ -145,13 +125,7 @@ __global__ void __launch_bounds__(kQT) k_unsharp_quads(const char* in, int64_t i
         if (k.cheap) {
           r[c] = unsharp_cheap_f32(ov[c], bv[c], k);
         } else if (!(k.a_exact && unsharp_front_f32(ov[c], bv[c], k, r[c])) && !unsharp_fast_f32(ov[c], bv[c], k, r[c])) {
-          const uint32_t slot = defer ? atomicAdd(&n_def, 1u) : kDeferCap;
-          if (slot < kDeferCap) {
-            seg[slot] = i * 4 + (I)c;
-            r[c] = blur == out ? bv[c] : ov[c];  // replaced by k_unsharp_deferred
-          } else {
-            r[c] = __double2float_rn(unsharp_f64((double)ov[c], (double)bv[c], k.amount, k.threshold));
-          }
+          r[c] = __double2float_rn(unsharp_f64((double)ov[c], (double)bv[c], k.amount, k.threshold));
         }
       }
       float4* const dq = reinterpret_cast<float4*>(out + ooff[h]) + qxs[h];
@@ -161,33 +135,6 @@ __global__ void __launch_bounds__(kQT) k_unsharp_quads(const char* in, int64_t i
         for (int c = 0; c < ncols[h]; ++c) reinterpret_cast<float*>(dq)[c] = r[c];
       }
     }
-  }
-  if (!defer) return;
-  __syncthreads();
-  if (threadIdx.x == 0) defer_n[blockIdx.x] = min(n_def, (uint32_t)kDeferCap);
-}
-
-// The voxels k_unsharp_quads deferred: block b takes segment b.
-template <typename I>
-__global__ void __launch_bounds__(kQT) k_unsharp_deferred(const char* in, int64_t ip1, int64_t ip2, const char* blur,
-                                                           int64_t bp1, int64_t bp2, char* out, int64_t op1,
-                                                           int64_t op2, I nq, I m1, const UnsharpConsts k,
-                                                           const I* defer, const uint32_t* defer_n) {
-  const uint32_t n = defer_n[blockIdx.x];
-  const I* const seg = defer + (size_t)blockIdx.x * kDeferCap;
-  for (uint32_t j = threadIdx.x; j < n; j += kQT) {
-    const I e = seg[j];
-    const I i = e >> 2;
-    const int c = (int)(e & 3);
-    int64_t off;
-    I qx;
-    quad_addr(i, nq, m1, ip1, ip2, off, qx);
-    const float o = reinterpret_cast<const float*>(in + off)[4 * (int64_t)qx + c];
-    quad_addr(i, nq, m1, bp1, bp2, off, qx);
-    const float b = reinterpret_cast<const float*>(blur + off)[4 * (int64_t)qx + c];
-    quad_addr(i, nq, m1, op1, op2, off, qx);
-    reinterpret_cast<float*>(out + off)[4 * (int64_t)qx + c] =
-        __double2float_rn(unsharp_f64((double)o, (double)b, k.amount, k.threshold));
   }
 }
 
@@ -219,16 +166,6 @@ template <typename I>
 itkg_status launch_quads(const char* ic, const int64_t* ip, const char* bc, const int64_t* bp, char* oc,
                          const int64_t* op, const int64_t* m, uint64_t total, unsigned blocks, const UnsharpConsts& k,
                          cudaStream_t s) {
-  void* scratch = nullptr;
-  I* defer = nullptr;
-  uint32_t* defer_n = nullptr;
-  if (!k.cheap && !k.a_exact) {
-    const size_t list_bytes = (size_t)blocks * kDeferCap * sizeof(I);
-    const itkg_status st = scratch_alloc(&scratch, list_bytes + (size_t)blocks * sizeof(uint32_t), s);
-    if (st != ITKG_SUCCESS) return st;
-    defer = static_cast<I*>(scratch);
-    defer_n = reinterpret_cast<uint32_t*>(static_cast<char*>(scratch) + list_bytes);
-  }
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
@@ -240,18 +177,9 @@ itkg_status launch_quads(const char* ic, const int64_t* ip, const char* bc, cons
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, k_unsharp_quads<I>, ic, ip[1], ip[2], bc, bp[1], bp[2], oc, op[1],
-                                           op[2], (I)((m[0] + 3) / 4), (I)m[0], (I)m[1], (I)total, k, defer, defer_n);
+                                           op[2], (I)((m[0] + 3) / 4), (I)m[0], (I)m[1], (I)total, k);
   note_launch("unsharp");
-  if (e != cudaSuccess) {
-    scratch_free(scratch, s);
-    return set_error(ITKG_ERROR_CUDA, "unsharp launch: %s", cudaGetErrorString(e));
-  }
-  if (!defer) return ITKG_SUCCESS;
-  k_unsharp_deferred<I><<<blocks, kQT, 0, s>>>(ic, ip[1], ip[2], bc, bp[1], bp[2], oc, op[1], op[2], (I)((m[0] + 3) / 4),
-                                               (I)m[1], k, defer, defer_n);
-  note_launch("unsharp_deferred");
-  scratch_free(scratch, s);
-  return ITKG_SUCCESS;
+  return e == cudaSuccess ? ITKG_SUCCESS : set_error(ITKG_ERROR_CUDA, "unsharp launch: %s", cudaGetErrorString(e));
 }
 
 }  // namespace
@@ -313,17 +241,14 @@ itkg_status launch_unsharp(int dtype, int comps, const void* in, const int64_t* 
                      m[0] <= INT32_MAX && m[1] <= UINT32_MAX && a16(in, ip[1], ip[2]) &&
                      a16(blur, bp[1], bp[2]) && a16(out, op[1], op[2]);
   if (quads) {
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const uint64_t total = (uint64_t)((m[0] + 3) / 4) * (uint64_t)m[1] * (uint64_t)m[2];
     // one full wave of resident blocks (each thread takes two quads per step)
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_unsharp_quads<uint32_t>, kQT, 0);
-    const uint64_t blocks =
-        std::min<uint64_t>((total + 2 * kQT - 1) / (2 * kQT), (uint64_t)std::max(sms, 1) * std::max(per_sm, 1));
-    // quad indices * 4 + 3 must fit the index type
-    const itkg_status st = 4 * (total + (uint64_t)blocks * kQT) < UINT32_MAX
+    int resident = 0;
+    itkg_status st = max_resident_ctas(reinterpret_cast<const void*>(k_unsharp_quads<uint32_t>), 0, kQT, &resident);
+    if (st != ITKG_SUCCESS) return st;
+    const uint64_t blocks = std::min<uint64_t>((total + 2 * kQT - 1) / (2 * kQT), (uint64_t)resident);
+    // quad indices a step past the end must fit the index type
+    st = 4 * (total + (uint64_t)blocks * kQT) < UINT32_MAX
                                ? launch_quads<uint32_t>(ic, ip, bc, bp, oc, op, m, total, (unsigned)blocks, k, s)
                                : launch_quads<uint64_t>(ic, ip, bc, bp, oc, op, m, total, (unsigned)blocks, k, s);
     if (st != ITKG_SUCCESS) return st;
