@@ -1283,13 +1283,21 @@ itkg_status itkg_unsharp_mask_generate_region(const itkg_image* input, const itk
       }
     }
   }
-  // otherwise the blur into the output image, then the point-wise step in place;
-  // an output that shares memory with the input gets a blur image of its own
+  // otherwise the blur into the output image, then the point-wise step in place.
+  // An output that shares memory with the input gets a blur image of its own,
+  // and so does one whose quads are not on 16-byte boundaries, which would be
+  // stored and read again element by element.
   itkg_image blur = dout;
-  {
+  if (st == ITKG_SUCCESS && !fused) {
     const char* const i0 = static_cast<const char*>(din.data);
     const char* const o0 = static_cast<const char*>(dout.data);
-    if (st == ITKG_SUCCESS && !fused && i0 < o0 + image_bytes(dout) && o0 < i0 + image_bytes(din)) {
+    bool own = i0 < o0 + image_bytes(dout) && o0 < i0 + image_bytes(din);
+    int64_t first = (int64_t)(uintptr_t)o0;
+    for (int d = 0; d < D; ++d) {
+      first += (requested->index[d] - dout.region.index[d]) * dout.pitch[d];
+      own = own || (d > 0 && dout.pitch[d] % 16 != 0);
+    }
+    if (own || first % 16 != 0) {
       blur.region = *requested;
       dense_layout(&blur, 16);
       st = scratch_alloc(&pblur, image_bytes(blur), s);
