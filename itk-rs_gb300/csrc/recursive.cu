@@ -84,7 +84,7 @@ struct RecLines {
   int32_t pad_;
   RecImage in, out;     // FIRST / LAST
   int64_t in_step, out_step;  // their strides along the axis
-  int32_t w0, w1;       // LAST: the requested samples of a line
+  int64_t w0, w1;       // LAST: the requested samples of a line
   int64_t lo[3], hi[3]; // LAST: the requested region, from the largest one's first voxel
   double B, a1, a2, a3;
 };
@@ -128,24 +128,24 @@ __global__ void __launch_bounds__(32) k_rec_lines(const __grid_constant__ RecLin
     c[0] = L - q * n0, c[1] = a.axis == 1 ? 0 : q, c[2] = a.axis == 1 ? q : 0;
   }
   if (CONTIG ? L >= n1 * n2 : L >= n0 * (a.axis == 1 ? n2 : n1)) return;
-  const int n = (int)(CONTIG ? n0 : a.axis == 1 ? n1 : n2);
+  const int64_t n = CONTIG ? n0 : a.axis == 1 ? n1 : n2;
   const int64_t s = CONTIG ? 1 : a.axis == 1 ? a.pitch : a.pitch * n1;
   double* const p = a.d + (c[2] * n1 + c[1]) * a.pitch + c[0];
   const int64_t is = a.in_step, os = a.out_step;
   const char* const ip = FIRST ? a.in.at + c[0] * a.in.p[0] + c[1] * a.in.p[1] + c[2] * a.in.p[2] : nullptr;
   char* const op = LAST ? a.out.at + c[0] * a.out.p[0] + c[1] * a.out.p[1] + c[2] * a.out.p[2] : nullptr;
-  int w0 = 0, w1 = 0;  // samples to write
+  int64_t w0 = 0, w1 = 0;  // samples to write
   if (LAST) {
     bool in = true;
 #pragma unroll
     for (int d = 0; d < 3; ++d) in = in && (d == a.axis || (c[d] >= a.lo[d] && c[d] < a.hi[d]));
     if (in) w0 = a.w0, w1 = a.w1;
   }
-  auto read = [&](int i, double (&v)[4]) {  // samples i .. i + 3 of the axis' input
-    const int m = min(4, n - i);
+  auto read = [&](int64_t i, double (&v)[4]) {  // samples i .. i + 3 of the axis' input
+    const int m = (int)min((int64_t)4, n - i);
     if constexpr (FIRST) {
 #pragma unroll
-      for (int k = 0; k < 4; ++k) v[k] = rec_read(ip + (int64_t)(i + min(k, m - 1)) * is, a.in.dtype);
+      for (int k = 0; k < 4; ++k) v[k] = rec_read(ip + (i + min(k, m - 1)) * is, a.in.dtype);
     } else {
       rec_load4<CONTIG>(p + i * s, s, m, v);
     }
@@ -153,9 +153,9 @@ __global__ void __launch_bounds__(32) k_rec_lines(const __grid_constant__ RecLin
   double v[4], nx[4];
   read(0, v);
   double y1 = v[0], y2 = y1, y3 = y1;  // steady state of the first sample
-  for (int i = 0; i < n; i += 4) {
+  for (int64_t i = 0; i < n; i += 4) {
     if (i + 4 < n) read(i + 4, nx);
-    const int m = min(4, n - i);
+    const int m = (int)min((int64_t)4, n - i);
     double o[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
@@ -175,11 +175,11 @@ __global__ void __launch_bounds__(32) k_rec_lines(const __grid_constant__ RecLin
   // group first
   y2 = y1;
   y3 = y1;
-  const int top = (n - 1) / 4 * 4;
-  rec_load4<CONTIG>(p + top * s, s, n - top, v);
-  for (int i = top; i >= 0; i -= 4) {
+  const int64_t top = (n - 1) / 4 * 4;
+  rec_load4<CONTIG>(p + top * s, s, (int)(n - top), v);
+  for (int64_t i = top; i >= 0; i -= 4) {
     if (i >= 4) rec_load4<CONTIG>(p + (i - 4) * s, s, 4, nx);
-    const int m = min(4, n - i);
+    const int m = (int)min((int64_t)4, n - i);
     double o[4];
 #pragma unroll
     for (int k = 3; k >= 0; --k) {
@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(32) k_rec_lines(const __grid_constant__ RecLin
     if constexpr (LAST) {
 #pragma unroll
       for (int k = 0; k < 4; ++k)
-        if (i + k >= w0 && i + k < w1) rec_write(op + (int64_t)(i + k) * os, a.out.dtype, o[k]);
+        if (i + k >= w0 && i + k < w1) rec_write(op + (i + k) * os, a.out.dtype, o[k]);
     } else {
       rec_store4<CONTIG>(p + i * s, s, m, o);
     }
@@ -382,7 +382,6 @@ itkg_status launch_recursive(const itkg_image& in, const itkg_region& largest, c
       a.lo[d] = requested.index[d] - g.lo[d];
       a.hi[d] = a.lo[d] + (int64_t)requested.size[d];
       if ((axis < 0 || d == axis) && g.n[d] > 1) axes[naxes++] = d;
-      if (g.n[d] > INT32_MAX / 2) return set_error(ITKG_ERROR_UNSUPPORTED, "axis %d is too long", d);
     } else {
       a.hi[d] = 1;
     }
@@ -415,7 +414,7 @@ itkg_status launch_recursive(const itkg_image& in, const itkg_region& largest, c
     a.axis = d;
     a.in_step = a.in.p[d];
     a.out_step = a.out.p[d];
-    a.w0 = (int32_t)a.lo[d], a.w1 = (int32_t)a.hi[d];
+    a.w0 = a.lo[d], a.w1 = a.hi[d];
     a.B = c[0], a.a1 = c[1], a.a2 = c[2], a.a3 = c[3];
     const int64_t lines = g.n[0] * g.n[1] * g.n[2] / g.n[d];
     const unsigned blocks = (unsigned)((lines + 31) / 32);
