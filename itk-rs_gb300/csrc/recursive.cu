@@ -79,7 +79,7 @@ __device__ __forceinline__ void rec_write(char* p, int dtype, double v) {
 struct RecLines {
   RecGeom g;
   double* d;            // scratch: sample (x, y, z) at (z n1 + y) pitch + x
-  int64_t pitch;        // doubles per row, a multiple of 4
+  int64_t pitch;        // doubles per row; even where rows are filtered (16-byte accesses)
   int32_t axis;
   int32_t pad_;
   RecImage in, out;     // FIRST / LAST
@@ -367,7 +367,7 @@ itkg_status launch_recursive(const itkg_image& in, const itkg_region& largest, c
   RecLines a;
   std::memset(&a, 0, sizeof a);
   a.g = g;
-  a.pitch = (g.n[0] + 3) / 4 * 4;
+  a.pitch = g.n[0] > 1 && axis <= 0 ? (g.n[0] + 1) / 2 * 2 : g.n[0];
   a.in.at = static_cast<char*>(in.data);
   a.out.at = static_cast<char*>(out.data);
   a.in.dtype = in.dtype;

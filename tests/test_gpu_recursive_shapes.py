@@ -2,6 +2,9 @@
 over: an axis beyond 2^30 samples, images a few columns wide (scratch rows),
 and outputs that overlap the input elsewhere than voxel on voxel."""
 import ctypes
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -9,6 +12,7 @@ import pytest
 import oracle
 
 pytestmark = pytest.mark.gpu
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 def test_an_axis_of_2_to_the_30(gpu):
@@ -29,3 +33,37 @@ def test_an_axis_of_2_to_the_30(gpu):
             gpu._abi.check(L.itkg_memcpy(got[y].ctypes.data, ctypes.c_void_p(out.c.data + y * out.c.pitch[1] + x0), 4096, 1, None))
         gpu._abi.check(L.itkg_stream_synchronize(None))
         assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("nx", [1, 2, 3, 5, 7])
+@pytest.mark.parametrize("axis", [None, 0, 1])
+def test_narrow_images(gpu, nx, axis):
+    x = np.random.default_rng(nx).standard_normal((9, 50, nx)).astype(np.float32)
+    dev = gpu.DeviceImage.from_host(gpu.Image(x))
+    got = gpu.RecursiveGaussianFilter(dev, 1.7, axis=axis).generate_region(dev.region).download()
+    want = oracle.recursive_gaussian_f32(x, 1.7, axis=-1 if axis is None else axis)
+    assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
+
+
+ONE_COLUMN = """
+import sys
+sys.path.insert(0, {root!r} + "/itk-rs_gb300")
+import itkg, torch
+n = 1 << 12
+region = itkg.Region((0, 0, 0), (1, 4, 4))
+warm = itkg.DeviceImage(region, itkg.U8)
+itkg.RecursiveGaussianFilter(warm, 2.0).generate_region(region)
+dev, free = itkg.DeviceImage(itkg.Region((0, 0, 0), (1, n, n)), itkg.U8), []
+for i in range(2):
+    torch.cuda.synchronize()
+    free.append(torch.cuda.mem_get_info()[0])
+    out = itkg.RecursiveGaussianFilter(dev, 2.0).generate_region(region)
+print(free[0] - free[1])
+"""
+
+
+def test_scratch_of_a_one_column_image(gpu):
+    """8 bytes of scratch a sample, 128 MiB for 2^24, not rows of four (512 MiB)."""
+    p = subprocess.run([sys.executable, "-c", ONE_COLUMN.format(root=ROOT)], capture_output=True, text=True, timeout=300)
+    assert p.returncode == 0, p.stderr
+    assert int(p.stdout.split()[-1]) < 320 << 20, p.stdout
