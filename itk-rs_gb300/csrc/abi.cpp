@@ -984,6 +984,25 @@ itkg_status itkg_yvv_coeffs(double sigma, double* coeffs_out) {
   return ITKG_SUCCESS;
 }
 
+// Whether the line passes would overwrite samples that they still have to read:
+// with fewer than two axes to filter, one kernel reads the input and writes the
+// output, which must then lie voxel on voxel or apart.
+static bool recursive_overlaps(const itkg_image& in, const itkg_image& out, const itkg_region& largest, int axis) {
+  if (in.location == ITKG_HOST || out.location == ITKG_HOST) return false;
+  const char* const i0 = static_cast<const char*>(in.data);
+  const char* const o0 = static_cast<const char*>(out.data);
+  if (!(i0 < o0 + image_bytes(out) && o0 < i0 + image_bytes(in))) return false;
+  int naxes = 0;
+  int64_t shift = o0 - i0;
+  bool same = dtype_size(in.dtype) == dtype_size(out.dtype);
+  for (int d = 0; d < in.dim; ++d) {
+    if ((axis < 0 || d == axis) && largest.size[d] > 1) ++naxes;
+    same = same && in.pitch[d] == out.pitch[d];
+    shift += (in.region.index[d] - out.region.index[d]) * in.pitch[d];
+  }
+  return naxes < 2 && !(same && shift == 0);
+}
+
 itkg_status itkg_recursive_gaussian_generate_region(const itkg_image* input, const itkg_region* largest,
                                                     const itkg_region* requested,
                                                     const itkg_recursive_params* params, itkg_image* output,
@@ -1018,7 +1037,7 @@ itkg_status itkg_recursive_gaussian_generate_region(const itkg_image* input, con
   void* pin = nullptr;
   void* pout = nullptr;
   itkg_status st = ITKG_SUCCESS;
-  if (host_in) {
+  if (host_in || recursive_overlaps(*input, *output, *largest, params->axis)) {
     din.location = ITKG_DEVICE;
     din.region = *largest;
     dense_layout(&din, 16);

@@ -67,3 +67,21 @@ def test_scratch_of_a_one_column_image(gpu):
     p = subprocess.run([sys.executable, "-c", ONE_COLUMN.format(root=ROOT)], capture_output=True, text=True, timeout=300)
     assert p.returncode == 0, p.stderr
     assert int(p.stdout.split()[-1]) < 320 << 20, p.stdout
+
+
+@pytest.mark.parametrize("axis,shift", [(0, 0), (0, 1), (0, 40), (1, 0), (1, 3), (1, 64 * 3)])
+def test_output_over_the_input(gpu, axis, shift):
+    """One filtered axis, the output `shift` samples further on in the input's memory."""
+    x = np.random.default_rng(shift).standard_normal((80, 64)).astype(np.float32)
+    big = gpu.DeviceImage(gpu.Region((0,), (80 * 64 + 256,)))
+    big.upload(np.concatenate([x.ravel(), np.zeros(256, np.float32)]))
+    L, im = gpu._abi.lib(), gpu.Image(x)
+    src, dst = im.to_c(), im.to_c()
+    for c, off in ((src, 0), (dst, 4 * shift)):
+        c.location, c.data = gpu._abi.DEVICE, big.c.data + off
+    f = gpu.RecursiveGaussianFilter(im, 2.0, axis=axis)
+    reg, prm = im.region.to_c(), f.params()
+    gpu._abi.check(L.itkg_recursive_gaussian_generate_region(ctypes.byref(src), ctypes.byref(reg), ctypes.byref(reg),
+                                                             ctypes.byref(prm), ctypes.byref(dst), None))
+    got = big.download()[shift:shift + 80 * 64].reshape(80, 64)
+    assert np.array_equal(got.view(np.uint32), oracle.recursive_gaussian_f32(x, 2.0, axis=axis).view(np.uint32))
