@@ -314,6 +314,13 @@ static itkg_status check_params(const itkg_gaussian_params* prm) {
   return ITKG_SUCCESS;
 }
 
+// Whether two images' buffers share memory.
+static bool overlap(const itkg_image& a, const itkg_image& b) {
+  const char* const a0 = static_cast<const char*>(a.data);
+  const char* const b0 = static_cast<const char*>(b.data);
+  return a0 < b0 + image_bytes(b) && b0 < a0 + image_bytes(a);
+}
+
 // Device-resident input and output.
 static void make_fused_geom(const itkg_image& in, const itkg_region& largest,
                             const itkg_region& requested, const itkg_gaussian_params& prm,
@@ -470,8 +477,10 @@ static itkg_status generate_device(const itkg_image& in, const itkg_region& larg
     // a megapixel (512^2, radius 9: 8.7 against 11.3 us, mostly launches); the
     // line passes beyond (1601 x 1067, radius 9, 3 components: 35 against 50 us,
     // the tiles' halo rows).
-    const bool tiles = plan.radii[0] < 8 ||
-                       (in.components == 1 && region_len(requested, D) <= (1ull << 20));
+    // A tile reads its neighbours' pixels, so an output over the input's memory
+    // takes the per-axis passes, whose last one reads scratch.
+    const bool tiles = !overlap(in, out) &&
+                       (plan.radii[0] < 8 || (in.components == 1 && region_len(requested, D) <= (1ull << 20)));
     if (D == 2 && tiles && prm.algorithm == ITKG_ALGO_AUTO && launch_tile2d_u8(g, w, s, /*dry_run=*/true) == ITKG_SUCCESS)
       return launch_tile2d_u8(g, w, s, false);
     if (prm.algorithm == ITKG_ALGO_FUSED)
@@ -989,11 +998,9 @@ itkg_status itkg_yvv_coeffs(double sigma, double* coeffs_out) {
 // output, which must then lie voxel on voxel or apart.
 static bool recursive_overlaps(const itkg_image& in, const itkg_image& out, const itkg_region& largest, int axis) {
   if (in.location == ITKG_HOST || out.location == ITKG_HOST) return false;
-  const char* const i0 = static_cast<const char*>(in.data);
-  const char* const o0 = static_cast<const char*>(out.data);
-  if (!(i0 < o0 + image_bytes(out) && o0 < i0 + image_bytes(in))) return false;
+  if (!overlap(in, out)) return false;
   int naxes = 0;
-  int64_t shift = o0 - i0;
+  int64_t shift = static_cast<const char*>(out.data) - static_cast<const char*>(in.data);
   bool same = dtype_size(in.dtype) == dtype_size(out.dtype);
   for (int d = 0; d < in.dim; ++d) {
     if ((axis < 0 || d == axis) && largest.size[d] > 1) ++naxes;
@@ -1308,10 +1315,8 @@ itkg_status itkg_unsharp_mask_generate_region(const itkg_image* input, const itk
   // stored and read again element by element.
   itkg_image blur = dout;
   if (st == ITKG_SUCCESS && !fused) {
-    const char* const i0 = static_cast<const char*>(din.data);
-    const char* const o0 = static_cast<const char*>(dout.data);
-    bool own = i0 < o0 + image_bytes(dout) && o0 < i0 + image_bytes(din);
-    int64_t first = (int64_t)(uintptr_t)o0;
+    bool own = overlap(din, dout);
+    int64_t first = (int64_t)(uintptr_t)dout.data;
     for (int d = 0; d < D; ++d) {
       first += (requested->index[d] - dout.region.index[d]) * dout.pitch[d];
       own = own || (d > 0 && dout.pitch[d] % 16 != 0);
