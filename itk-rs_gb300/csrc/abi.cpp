@@ -314,13 +314,6 @@ static itkg_status check_params(const itkg_gaussian_params* prm) {
   return ITKG_SUCCESS;
 }
 
-// Whether two images' buffers share memory.
-static bool overlap(const itkg_image& a, const itkg_image& b) {
-  const char* const a0 = static_cast<const char*>(a.data);
-  const char* const b0 = static_cast<const char*>(b.data);
-  return a0 < b0 + image_bytes(b) && b0 < a0 + image_bytes(a);
-}
-
 // Device-resident input and output.
 static void make_fused_geom(const itkg_image& in, const itkg_region& largest,
                             const itkg_region& requested, const itkg_gaussian_params& prm,

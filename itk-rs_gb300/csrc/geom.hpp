@@ -164,4 +164,11 @@ inline size_t image_bytes(const itkg_image& im) {
 
 // Copy `reg` between two images (any locations) with 2-D copies per slice, or
 
+// Whether two images' buffers share memory.
+inline bool overlap(const itkg_image& a, const itkg_image& b) {
+  const char* const a0 = static_cast<const char*>(a.data);
+  const char* const b0 = static_cast<const char*>(b.data);
+  return a0 < b0 + image_bytes(b) && b0 < a0 + image_bytes(a);
+}
+
 }  // namespace itkg

@@ -301,6 +301,9 @@ extern "C" itkg_status itkg_gaussian_scale_stack_loss_vjp(
   double* dsig = dloss + 1;
   int64_t nloss = 0;
   const bool on_dev = flags & ITKG_VJP_SIGMA_BAR_ON_DEVICE;
+  // the two-pass VJP writes xbar before its last read of x; the per-axis chain
+  // of a single level has read x by then
+  const bool x_in_xbar = xbar && overlap(*x, *xbar);
   int fast_levels = 0;
   for (int l = 0; l < nlevels; ++l) {
     const AxisCoeffs* c = &coeffs[(size_t)l * kMaxDim];
@@ -319,7 +322,7 @@ extern "C" itkg_status itkg_gaussian_scale_stack_loss_vjp(
     v.acc_sigma = false;
     for (int d = 0; d < x->dim; ++d) v.w[d] = c[d].w.data(), v.dw[d] = c[d].dw.data(), v.radius[d] = (int)c[d].r;
     int blocks = nb;
-    if (x->dim == 3 && (x->region.size[0] % 4 == 0 || n >= kRaggedTwoPass) &&
+    if (x->dim == 3 && (x->region.size[0] % 4 == 0 || n >= kRaggedTwoPass) && !x_in_xbar &&
         launch_vjp_two_pass(v, s, true) == ITKG_SUCCESS) {
       itkg_gaussian_params p;
       std::memset(&p, 0, sizeof p);
