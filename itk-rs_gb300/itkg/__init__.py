@@ -109,8 +109,8 @@ class Region:
                 self.__dict__["_c_struct"] = r
         return r
 
-    def __reduce__(self):
-        return Region, (self.index, self.size)
+    def __getstate__(self):  # what is copied and pickled: everything but the cached struct
+        return {k: v for k, v in self.__dict__.items() if k != "_c_struct"}
 
     @staticmethod
     def from_c(r: itkg_region, dim: int) -> "Region":
