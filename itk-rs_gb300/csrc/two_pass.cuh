@@ -564,48 +564,38 @@ __global__ void __launch_bounds__(256, RZ <= (REF ? 6 : 8) ? 2 : 1) k_z_pass(con
   // the next call's x-y grid may be scheduled now; it waits for this grid
   // before its first global memory access
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+  // block: 32 rows of a T tile, the blocks of a tile one after another as the
+  // x-y pass walks its tiles; blocks of the last tile row that hold no requested
+  // row are not counted.  This thread's quad: row w / 8 of the tile, columns
+  // 4 (w % 8) .. + 3.  The first block's place is found before the wait, under
+  // the x-y pass's last CTAs: FMA rounding, the call, with every place found after
+  // it and here, RZ = 4 on 192^3 19.9 and 19.8 us, RZ = 10 on 256^3 64.4 and 63.6;
+  // a 64-bit block index for FMA rounding alone took 22.0 and 67.0 (47.5 against
+  // 47.6 for RZ = 6 on 256^3).
+  const int tile_q = a.tile_rows * (kTileX / 4);  // quads per tile
+  int64_t u = u_begin;
+  int tly = 0, tix = 0, w = 0, zs = 0;
+  auto place = [&]() {
+    const int blk = (int)(u / a.nz);
+    zs = (int)(u - (int64_t)blk * a.nz);
+    const int bpt = a.tile_rows / 32, nrb = (a.ny + 31) / 32;
+    tly = blk / (a.ntx * bpt);
+    const int in_row = blk - tly * a.ntx * bpt;
+    const int nb = min(bpt, nrb - tly * bpt);  // blocks of this row's tiles
+    tix = in_row / nb;
+    w = (in_row - tix * nb) * C::QB + tid;
+  };
+  place();
   // T is written by the x-y grid this launch depends on (programmatic dependent
   // launch): wait for it to complete and its writes to be visible
   asm volatile("griddepcontrol.wait;\n" ::: "memory");
 
-  for (int64_t u = u_begin; u < u_end;) {
-    const int64_t blk = u / a.nz;
-    const int zs = (int)(u - blk * a.nz);
+  for (bool first = true; u < u_end; first = false) {
+    if (!first) place();
     const int64_t zrem = zs + (u_end - u);
     const int ze = zrem < a.nz ? (int)zrem : a.nz;
     u += ze - zs;
-    // block: 32 rows of a T tile, the blocks of a tile one after another as the
-    // x-y pass walks its tiles; blocks of the last tile row that hold no requested
-    // row are not counted.  This thread's quad: T tile `tl`, quad w (row w / 8,
-    // columns 4 (w % 8) .. + 3).  Two forms of the same numbering, for the
-    // registers that the march is left with: FMA 256^3, RZ = 6, the call 47.6 us
-    // in 64 bits and 47.7 in 32; reference rounding, 197 x 233 x 189, RZ = 5, 47.9
-    // and 47.3, and 192^3 in the unsharp mask 60.0 and 58.6.
-    const int tile_q = a.tile_rows * (kTileX / 4);  // quads per tile
-    int64_t tl;
-    int w, tix, tly;
-    if constexpr (REF) {
-      const int bpt = a.tile_rows / 32, nrb = (a.ny + 31) / 32;
-      tly = (int)blk / (a.ntx * bpt);
-      const int in_row = (int)blk - tly * a.ntx * bpt;
-      const int nb = min(bpt, nrb - tly * bpt);  // blocks of this row's tiles
-      tix = in_row / nb;
-      tl = (int64_t)tly * a.ntx + tix;
-      w = (in_row - tix * nb) * C::QB + tid;
-    } else {
-      const int64_t bpt = a.tile_rows / 32, full = a.ny / a.tile_rows * bpt * a.ntx;
-      int64_t blk_t = blk;  // counting every block of the last tile row
-      if (blk >= full) {
-        const int64_t nb = (a.ny % a.tile_rows + 31) / 32, t = (blk - full) / nb;
-        blk_t = full + t * bpt + (blk - full - t * nb);
-      }
-      const int64_t q = blk_t * C::QB + tid;
-      tl = q / tile_q;
-      w = (int)(q - tl * tile_q);
-      const int64_t ty = tl / a.ntx;
-      tix = (int)(tl - ty * a.ntx);
-      tly = (int)ty;
-    }
+    const int64_t tl = (int64_t)tly * a.ntx + tix;
     const int cx = tix * kTileX + 4 * (w & (kTileX / 4 - 1));  // first column
     const int cy = tly * a.tile_rows + w / (kTileX / 4);       // row
     if (cy >= a.ny || cx >= a.nx) continue;  // no barriers in this kernel: idle threads just skip

@@ -69,12 +69,14 @@ def test_scratch_of_a_one_column_image(gpu):
     assert int(p.stdout.split()[-1]) < 320 << 20, p.stdout
 
 
-@pytest.mark.parametrize("axis,shift", [(0, 0), (0, 1), (0, 40), (1, 0), (1, 3), (1, 64 * 3)])
-def test_output_over_the_input(gpu, axis, shift):
+# (the last two: more lines than the device holds threads for, the output over lines of later blocks)
+@pytest.mark.parametrize("shape,axis,shift", [((80, 64), 0, 0), ((80, 64), 0, 1), ((80, 64), 1, 0), ((80, 64), 1, 192),
+                                              ((600000, 8), 0, 8 * 250000), ((6, 700000), 1, 300000)])
+def test_output_over_the_input(gpu, shape, axis, shift):
     """One filtered axis, the output `shift` samples further on in the input's memory."""
-    x = np.random.default_rng(shift).standard_normal((80, 64)).astype(np.float32)
-    big = gpu.DeviceImage(gpu.Region((0,), (80 * 64 + 256,)))
-    big.upload(np.concatenate([x.ravel(), np.zeros(256, np.float32)]))
+    x = np.random.default_rng(shift).standard_normal(shape).astype(np.float32)
+    big = gpu.DeviceImage(gpu.Region((0,), (x.size + shift,)))
+    big.upload(np.concatenate([x.ravel(), np.zeros(shift, np.float32)]))
     L, im = gpu._abi.lib(), gpu.Image(x)
     src, dst = im.to_c(), im.to_c()
     for c, off in ((src, 0), (dst, 4 * shift)):
@@ -83,5 +85,5 @@ def test_output_over_the_input(gpu, axis, shift):
     reg, prm = im.region.to_c(), f.params()
     gpu._abi.check(L.itkg_recursive_gaussian_generate_region(ctypes.byref(src), ctypes.byref(reg), ctypes.byref(reg),
                                                              ctypes.byref(prm), ctypes.byref(dst), None))
-    got = big.download()[shift:shift + 80 * 64].reshape(80, 64)
+    got = big.download()[shift:].reshape(shape)
     assert np.array_equal(got.view(np.uint32), oracle.recursive_gaussian_f32(x, 2.0, axis=axis).view(np.uint32))
