@@ -1283,9 +1283,13 @@ itkg_status itkg_unsharp_mask_generate_region(const itkg_image* input, const itk
   // directly.  Reference rounding from kUnsharpSplit voxels on: the exact step
   // holds the z kernel's few warps up more than a second trip through memory
   // costs, so the blur goes to the output image and the point-wise kernels turn
-  // it into the result in place.  192^3, sigma 1.5, the call: 74.7 us in one,
-  // 65.7 us split (amount 0.5; 89 and 75.8 us with 0.37); 128^3: 22.7 and 30 us.
-  constexpr uint64_t kUnsharpSplit = 1ull << 22;
+  // it into the result in place.  The call in one and split, us, smooth / white
+  // data, amount 0.37 at sigma 1.5: 96^3 15.7 / 13.6 and 17.7 / 14.8, 104^3 25.0 /
+  // 20.8 and 22.1 / 19.4, 128^3 27.3 / 22.7 and 26.6 / 22.4, 192^3 70.9 / 57.6 and
+  // 65.8 / 57.9; amount 0.5 at sigma 3: 96^3 19.6 / 23.0 and 20.4 / 21.4, 192^3
+  // 76.5 / 106.8 and 80.4 / 85.0.  Amount 0.5 on smooth data at sigma 1.5 alone
+  // is ahead in one: 128^3 20.8 and 22.1, 192^3 51.5 and 57.3.
+  constexpr uint64_t kUnsharpSplit = 960ull << 10;
   const bool split = params->rounding == ITKG_ROUND_REFERENCE && region_len(*requested, D) >= kUnsharpSplit;
   bool fused = false;
   if (st == ITKG_SUCCESS && !split && D == 3 && input->dtype == ITKG_F32 && input->components == 1) {
