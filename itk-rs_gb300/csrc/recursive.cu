@@ -4,10 +4,12 @@
 // region to f64 (P::to_f64), runs on every line along each axis a causal then
 // an anticausal pass in place (recursive_gaussian.rs:56-130), and converts the
 // requested region back (P::from_f64).  Here:
-//   k_rec_load   the largest region -> a dense f64 scratch image
-//   k_rec_lines  one thread per line: the causal pass, then the anticausal pass
-//   k_rec_store  the requested region -> the output (f32: round to nearest; u8:
-//                round half away from zero, clamp to [0, 255], NaN -> 0)
+//   k_rec_lines  one thread per line: the causal pass, then the anticausal pass,
+//                in an f64 scratch image; the first axis' kernel converts as it
+//                reads the input, the last one's as it writes the requested
+//                region (f32: round to nearest; u8: round half away from zero,
+//                clamp to [0, 255], NaN -> 0)
+//   k_rec_copy   the requested region alone, where no axis is filtered
 // Reference rounding rounds every product and sum separately in the
 // reference's order, bit for bit; FMA rounding uses fused multiply-adds (f64
 // throughout either way: an f32 recursion drifts past 1e-5 of the reference
@@ -115,8 +117,10 @@ __device__ __forceinline__ void rec_store4(double* p, int64_t s, int n, const do
 }
 
 // One line per thread.  axis 0: lines are rows (CONTIG); axis 1: stride pitch;
-// axis 2: stride n1 pitch.
-template <bool REF, bool FIRST, bool LAST, bool CONTIG>
+// axis 2: stride n1 pitch.  I: the type that counts a line's samples; 64 bits
+// only for lines beyond 2^30 (256^3, three axes, reference and FMA rounding: 1501
+// and 871 us in 32 bits, 1580 and 1053 in 64).
+template <typename I, bool REF, bool FIRST, bool LAST, bool CONTIG>
 __global__ void __launch_bounds__(32) k_rec_lines(const __grid_constant__ RecLines a) {
   const int64_t L = (int64_t)blockIdx.x * 32 + threadIdx.x;
   const int64_t n0 = a.g.n[0], n1 = a.g.n[1], n2 = a.g.n[2];
@@ -128,24 +132,24 @@ __global__ void __launch_bounds__(32) k_rec_lines(const __grid_constant__ RecLin
     c[0] = L - q * n0, c[1] = a.axis == 1 ? 0 : q, c[2] = a.axis == 1 ? q : 0;
   }
   if (CONTIG ? L >= n1 * n2 : L >= n0 * (a.axis == 1 ? n2 : n1)) return;
-  const int64_t n = CONTIG ? n0 : a.axis == 1 ? n1 : n2;
+  const I n = (I)(CONTIG ? n0 : a.axis == 1 ? n1 : n2);
   const int64_t s = CONTIG ? 1 : a.axis == 1 ? a.pitch : a.pitch * n1;
   double* const p = a.d + (c[2] * n1 + c[1]) * a.pitch + c[0];
   const int64_t is = a.in_step, os = a.out_step;
   const char* const ip = FIRST ? a.in.at + c[0] * a.in.p[0] + c[1] * a.in.p[1] + c[2] * a.in.p[2] : nullptr;
   char* const op = LAST ? a.out.at + c[0] * a.out.p[0] + c[1] * a.out.p[1] + c[2] * a.out.p[2] : nullptr;
-  int64_t w0 = 0, w1 = 0;  // samples to write
+  I w0 = 0, w1 = 0;  // samples to write
   if (LAST) {
     bool in = true;
 #pragma unroll
     for (int d = 0; d < 3; ++d) in = in && (d == a.axis || (c[d] >= a.lo[d] && c[d] < a.hi[d]));
-    if (in) w0 = a.w0, w1 = a.w1;
+    if (in) w0 = (I)a.w0, w1 = (I)a.w1;
   }
-  auto read = [&](int64_t i, double (&v)[4]) {  // samples i .. i + 3 of the axis' input
-    const int m = (int)min((int64_t)4, n - i);
+  auto read = [&](I i, double (&v)[4]) {  // samples i .. i + 3 of the axis' input
+    const int m = (int)min((I)4, n - i);
     if constexpr (FIRST) {
 #pragma unroll
-      for (int k = 0; k < 4; ++k) v[k] = rec_read(ip + (i + min(k, m - 1)) * is, a.in.dtype);
+      for (int k = 0; k < 4; ++k) v[k] = rec_read(ip + (int64_t)(i + min(k, m - 1)) * is, a.in.dtype);
     } else {
       rec_load4<CONTIG>(p + i * s, s, m, v);
     }
@@ -153,9 +157,9 @@ __global__ void __launch_bounds__(32) k_rec_lines(const __grid_constant__ RecLin
   double v[4], nx[4];
   read(0, v);
   double y1 = v[0], y2 = y1, y3 = y1;  // steady state of the first sample
-  for (int64_t i = 0; i < n; i += 4) {
+  for (I i = 0; i < n; i += 4) {
     if (i + 4 < n) read(i + 4, nx);
-    const int m = (int)min((int64_t)4, n - i);
+    const int m = (int)min((I)4, n - i);
     double o[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
@@ -175,11 +179,11 @@ __global__ void __launch_bounds__(32) k_rec_lines(const __grid_constant__ RecLin
   // group first
   y2 = y1;
   y3 = y1;
-  const int64_t top = (n - 1) / 4 * 4;
+  const I top = (n - 1) / 4 * 4;
   rec_load4<CONTIG>(p + top * s, s, (int)(n - top), v);
-  for (int64_t i = top; i >= 0; i -= 4) {
+  for (I i = top; i >= 0; i -= 4) {
     if (i >= 4) rec_load4<CONTIG>(p + (i - 4) * s, s, 4, nx);
-    const int m = (int)min((int64_t)4, n - i);
+    const int m = (int)min((I)4, n - i);
     double o[4];
 #pragma unroll
     for (int k = 3; k >= 0; --k) {
@@ -196,12 +200,25 @@ __global__ void __launch_bounds__(32) k_rec_lines(const __grid_constant__ RecLin
     if constexpr (LAST) {
 #pragma unroll
       for (int k = 0; k < 4; ++k)
-        if (i + k >= w0 && i + k < w1) rec_write(op + (i + k) * os, a.out.dtype, o[k]);
+        if (i + k >= w0 && i + k < w1) rec_write(op + (int64_t)(i + k) * os, a.out.dtype, o[k]);
     } else {
       rec_store4<CONTIG>(p + i * s, s, m, o);
     }
   }
 }
+
+using RecFn = void (*)(const RecLines);
+template <typename I>
+const RecFn kRecFns[2][2][2][2] = {  // [ref][first][last][axis 0]
+    {{{k_rec_lines<I, false, false, false, false>, k_rec_lines<I, false, false, false, true>},
+      {k_rec_lines<I, false, false, true, false>, k_rec_lines<I, false, false, true, true>}},
+     {{k_rec_lines<I, false, true, false, false>, k_rec_lines<I, false, true, false, true>},
+      {k_rec_lines<I, false, true, true, false>, k_rec_lines<I, false, true, true, true>}}},
+    {{{k_rec_lines<I, true, false, false, false>, k_rec_lines<I, true, false, false, true>},
+      {k_rec_lines<I, true, false, true, false>, k_rec_lines<I, true, false, true, true>}},
+     {{k_rec_lines<I, true, true, false, false>, k_rec_lines<I, true, true, false, true>},
+      {k_rec_lines<I, true, true, true, false>, k_rec_lines<I, true, true, true, true>}}}};
+constexpr int64_t kMaxInt32Line = 1 << 30;  // i + 4 stays below 2^31
 
 // No axis to filter: the requested region, converted and converted back.
 __global__ void __launch_bounds__(kT) k_rec_copy(RecImage in, RecImage out, int64_t r0, int64_t r1, int64_t r2, int64_t m0,
@@ -397,16 +414,6 @@ itkg_status launch_recursive(const itkg_image& in, const itkg_region& largest, c
     if (st != ITKG_SUCCESS) return st;
     a.d = buf;
   }
-  using Fn = void (*)(const RecLines);
-  static const Fn fns[2][2][2][2] = {  // [ref][first][last][axis 0]
-      {{{k_rec_lines<false, false, false, false>, k_rec_lines<false, false, false, true>},
-        {k_rec_lines<false, false, true, false>, k_rec_lines<false, false, true, true>}},
-       {{k_rec_lines<false, true, false, false>, k_rec_lines<false, true, false, true>},
-        {k_rec_lines<false, true, true, false>, k_rec_lines<false, true, true, true>}}},
-      {{{k_rec_lines<true, false, false, false>, k_rec_lines<true, false, false, true>},
-        {k_rec_lines<true, false, true, false>, k_rec_lines<true, false, true, true>}},
-       {{k_rec_lines<true, true, false, false>, k_rec_lines<true, true, false, true>},
-        {k_rec_lines<true, true, true, false>, k_rec_lines<true, true, true, true>}}}};
   for (int i = 0; i < naxes; ++i) {
     const int d = axes[i];
     double c[4];
@@ -418,6 +425,7 @@ itkg_status launch_recursive(const itkg_image& in, const itkg_region& largest, c
     a.B = c[0], a.a1 = c[1], a.a2 = c[2], a.a3 = c[3];
     const int64_t lines = g.n[0] * g.n[1] * g.n[2] / g.n[d];
     const unsigned blocks = (unsigned)((lines + 31) / 32);
+    const auto& fns = g.n[d] > kMaxInt32Line ? kRecFns<int64_t> : kRecFns<int>;
     fns[ref ? 1 : 0][i == 0][i + 1 == naxes][d == 0]<<<blocks, 32, 0, s>>>(a);
     note_launch(ref ? "recursive_lines_f64" : "recursive_lines_f64_fma");
   }
