@@ -9,7 +9,8 @@
 //                reads the input, the last one's as it writes the requested
 //                region (f32: round to nearest; u8: round half away from zero,
 //                clamp to [0, 255], NaN -> 0)
-//   k_rec_copy   the requested region alone, where no axis is filtered
+//   k_rec_copy   conversions alone: the requested region where no axis is
+//                filtered, and both ways around the passes of a few lines
 // Reference rounding rounds every product and sum separately in the
 // reference's order, bit for bit; FMA rounding uses fused multiply-adds (f64
 // throughout either way: an f32 recursion drifts past 1e-5 of the reference
@@ -220,15 +221,22 @@ const RecFn kRecFns[2][2][2][2] = {  // [ref][first][last][axis 0]
       {k_rec_lines<I, true, true, true, false>, k_rec_lines<I, true, true, true, true>}}}};
 constexpr int64_t kMaxInt32Line = 1 << 30;  // i + 4 stays below 2^31
 
-// No axis to filter: the requested region, converted and converted back.
+// Samples r .. r + m - 1 of the largest region, converted: between the images
+// where no axis is filtered, to and from scratch (kRecF64) where conversions
+// stay out of the line kernels.
+constexpr int kRecF64 = -1;
 __global__ void __launch_bounds__(kT) k_rec_copy(RecImage in, RecImage out, int64_t r0, int64_t r1, int64_t r2, int64_t m0,
                                                   int64_t m1, int64_t m2) {
   const int64_t i = (int64_t)blockIdx.x * kT + threadIdx.x;
   if (i >= m0) return;
   for (int64_t k = blockIdx.z; k < m2; k += gridDim.z)
-    for (int64_t j = blockIdx.y; j < m1; j += gridDim.y)
-      rec_write(out.at + (r0 + i) * out.p[0] + (r1 + j) * out.p[1] + (r2 + k) * out.p[2], out.dtype,
-                rec_read(in.at + (r0 + i) * in.p[0] + (r1 + j) * in.p[1] + (r2 + k) * in.p[2], in.dtype));
+    for (int64_t j = blockIdx.y; j < m1; j += gridDim.y) {
+      const char* const p = in.at + (r0 + i) * in.p[0] + (r1 + j) * in.p[1] + (r2 + k) * in.p[2];
+      char* const q = out.at + (r0 + i) * out.p[0] + (r1 + j) * out.p[1] + (r2 + k) * out.p[2];
+      const double v = in.dtype == kRecF64 ? *reinterpret_cast<const double*>(p) : rec_read(p, in.dtype);
+      if (out.dtype == kRecF64) *reinterpret_cast<double*>(q) = v;
+      else rec_write(q, out.dtype, v);
+    }
 }
 
 // The derivative users (edges.rs:686-950): stencils on the smoothed image `s`
@@ -405,14 +413,31 @@ itkg_status launch_recursive(const itkg_image& in, const itkg_region& largest, c
   }
   itkg_status st = ITKG_SUCCESS;
   double* buf = nullptr;
-  if (naxes == 0) {
-    k_rec_copy<<<grid3(a.hi[0] - a.lo[0], a.hi[1] - a.lo[1], a.hi[2] - a.lo[2]), kT, 0, s>>>(
-        a.in, a.out, a.lo[0], a.lo[1], a.lo[2], a.hi[0] - a.lo[0], a.hi[1] - a.lo[1], a.hi[2] - a.lo[2]);
+  auto copy = [&](const RecImage& from, const RecImage& to, const int64_t* lo, const int64_t* hi) {
+    k_rec_copy<<<grid3(hi[0] - lo[0], hi[1] - lo[1], hi[2] - lo[2]), kT, 0, s>>>(from, to, lo[0], lo[1], lo[2], hi[0] - lo[0],
+                                                                              hi[1] - lo[1], hi[2] - lo[2]);
     note_launch("recursive_copy");
+  };
+  RecImage scratch;
+  std::memset(&scratch, 0, sizeof scratch);
+  const int64_t none[3] = {0, 0, 0};
+  // One axis of few lines runs at the latency of its own f64 chain, which the
+  // conversions on the same pipe hold up: they run apart, over the whole image.
+  // (Up to four warps; they share no f64 pipe.)  30000 samples in one line,
+  // reference rounding: 17.2 ms with them in the line kernel, 14.4 apart.
+  const bool apart = naxes == 1 && g.n[0] * g.n[1] * g.n[2] / g.n[axes[0]] <= 128;
+  if (naxes == 0) {
+    copy(a.in, a.out, a.lo, a.hi);
   } else {
     st = scratch_alloc(reinterpret_cast<void**>(&buf), (size_t)(a.pitch * g.n[1] * g.n[2]) * sizeof(double), stream);
     if (st != ITKG_SUCCESS) return st;
     a.d = buf;
+    scratch.at = reinterpret_cast<char*>(buf);
+    scratch.dtype = kRecF64;
+    scratch.p[0] = sizeof(double);
+    scratch.p[1] = a.pitch * (int64_t)sizeof(double);
+    scratch.p[2] = scratch.p[1] * g.n[1];
+    if (apart) copy(a.in, scratch, none, g.n);
   }
   for (int i = 0; i < naxes; ++i) {
     const int d = axes[i];
@@ -426,9 +451,10 @@ itkg_status launch_recursive(const itkg_image& in, const itkg_region& largest, c
     const int64_t lines = g.n[0] * g.n[1] * g.n[2] / g.n[d];
     const unsigned blocks = (unsigned)((lines + 31) / 32);
     const auto& fns = g.n[d] > kMaxInt32Line ? kRecFns<int64_t> : kRecFns<int>;
-    fns[ref ? 1 : 0][i == 0][i + 1 == naxes][d == 0]<<<blocks, 32, 0, s>>>(a);
+    fns[ref ? 1 : 0][i == 0 && !apart][i + 1 == naxes && !apart][d == 0]<<<blocks, 32, 0, s>>>(a);
     note_launch(ref ? "recursive_lines_f64" : "recursive_lines_f64_fma");
   }
+  if (apart) copy(scratch, a.out, a.lo, a.hi);
   {
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) st = set_error(ITKG_ERROR_CUDA, "recursive gaussian launch: %s", cudaGetErrorString(e));

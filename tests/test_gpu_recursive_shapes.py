@@ -87,3 +87,20 @@ def test_output_over_the_input(gpu, shape, axis, shift):
                                                              ctypes.byref(prm), ctypes.byref(dst), None))
     got = big.download()[shift:].reshape(shape)
     assert np.array_equal(got.view(np.uint32), oracle.recursive_gaussian_f32(x, 2.0, axis=axis).view(np.uint32))
+
+
+@pytest.mark.parametrize("shape,axis", [((257,), None), ((4,), 0), ((300, 128), 1), ((300, 129), 1), ((128, 71), 0), ((129, 71), 0),
+                                        ((8, 16, 40), 0), ((8, 17, 40), 0), ((61, 8, 16), 2)])
+@pytest.mark.parametrize("dtype", [np.float32, np.uint8, np.int16])
+def test_few_lines_of_one_axis(gpu, shape, axis, dtype):
+    """Both sides of the 128 lines up to which the conversions run apart; whole images and sub-regions."""
+    rng = np.random.default_rng(sum(shape))
+    x = rng.integers(0, 256, shape).astype(dtype) if dtype != np.float32 else rng.standard_normal(shape).astype(dtype)
+    f64 = oracle.recursive_gaussian_f64(x.astype(np.float64), 1.9, axis=-1 if axis is None else axis)
+    want = oracle.from_f64_u8(f64) if dtype == np.uint8 else f64.astype(np.float32)
+    dev = gpu.DeviceImage.from_host(gpu.Image(x))
+    f = gpu.RecursiveGaussianFilter(dev, 1.9, axis=axis)
+    for at, size in [((0,) * x.ndim, tuple(reversed(shape))), (tuple(n // 3 for n in reversed(shape)), tuple((n + 3) // 4 for n in reversed(shape)))]:
+        got = f.generate_region(gpu.Region(at, size)).download()
+        sl = tuple(slice(at[d], at[d] + size[d]) for d in reversed(range(x.ndim)))
+        assert got.dtype == want.dtype and np.array_equal(got.view(np.uint8), np.ascontiguousarray(want[sl]).view(np.uint8))
