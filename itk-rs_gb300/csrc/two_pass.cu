@@ -199,12 +199,15 @@ itkg_status launch_two_pass(const FusedGeom& g, const float* const w[kMaxDim], v
   // 192 x 64 x 128: 12.1 and 11.8 / 17.4 and 15.2 / 17.3 and 15.1; more tiles of
   // 64 rows than one gain 3 % at best (ny 320, radius 6) and lose 5 (radius 2).
   // The fixed part: 192 x 430 x 128, radius 2, FMA: 4 tiles of 128 rows 34.5 us,
-  // 5 of 96 37.1.
+  // 5 of 96 37.1.  From f32, 96 rows have to cost 3 % less: where they cost 0 to 3 %
+  // less (400 to 480 rows) they were 1 % slower on average (420 rows, radius 5, RZ = 1,
+  // FMA: 22.5 us at 128, 25.0 at 96), from i16 2.5 % faster.
   if (g.radius[0] <= 8 && (u8p || g.in_dtype == ITKG_F32 || g.in_dtype == ITKG_I16)) {
     const int64_t h = g.req_size[1], r = g.radius[0];
     const int64_t fixed = (u8p || g.rounding == ITKG_ROUND_REFERENCE ? 128 : 256) / (r + 1);
     auto cost = [&](int64_t ty) { return (h + ty - 1) / ty * (2 * ty + 2 * r + fixed); };
-    const int rows = h <= 64 ? 64 : cost(96) < cost(128) ? 96 : 128;
+    const int64_t margin = !u8p && g.in_dtype == ITKG_F32 ? 97 : 100;
+    const int rows = h <= 64 ? 64 : 100 * cost(96) < margin * cost(128) ? 96 : 128;
     if (rows != 128)
       e = (u8p                        ? twopass::xy_rows_u8p(rows)
            : g.in_dtype == ITKG_F32 ? twopass::xy_rows_f32(rows)
